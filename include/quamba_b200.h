@@ -72,7 +72,10 @@ int qb_read_device_status(void* stream);
  *   (csrc/causal_conv1d/quant_causal_conv1d.cpp:77-164, :168-226).
  * y = silu( scale_w*scale_x * sum_w w[c,w] x[c, l-(W-1-w)] + scale_b*bias[c] ),
  * q_y = clamp(roundf(y / scale_out)).  x (B, D, L) with either L or D contiguous
- * (x_sl == 1 or x_sd == 1); out has the same strides as x.  width 2..4.
+ * (x_sl == 1 or x_sd == 1); out is contiguous in the same dimension as x.  width 2..4.
+ * conv_state (nullable, here and in the Quamba2 form): receives the last four inputs of every channel, oldest first and
+ * zeros before the start of the sequence, element (b, c, w) at b*state_sb + c*state_sd + w*state_sw: the window a decode
+ * step continues from.
  * ------------------------------------------------------------------------------------------ */
 typedef struct {
   const int8_t* x;
@@ -94,6 +97,10 @@ typedef struct {
   float scale_out;
   float scale_b;
   int32_t silu;
+  int8_t* conv_state;
+  int64_t state_sb;
+  int64_t state_sd;
+  int64_t state_sw;
 } qb_conv1d_fwd_args;
 int qb_causal_conv1d_fwd(const qb_conv1d_fwd_args* a, void* stream);
 
@@ -167,6 +174,10 @@ typedef struct {
   float scale_bB;
   float scale_bC;
   int32_t silu;
+  int8_t* conv_state;
+  int64_t state_sb;
+  int64_t state_sd;
+  int64_t state_sw;
 } qb_quamba2_conv1d_fwd_args;
 int qb_quamba2_conv1d_fwd(const qb_quamba2_conv1d_fwd_args* a, void* stream);
 

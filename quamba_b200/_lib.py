@@ -1,4 +1,5 @@
-"""ctypes binding of libquamba_b200.so.
+"""Loads the two native libraries: ctypes binding of libquamba_b200.so (the C ABI), and ``_native`` (the CPython extension the
+operator functions and layers call; csrc/binding.cpp).
 
 The argument structs are generated from ``include/quamba_b200.h`` at import time (the
 header keeps one ``type name;`` field per line for exactly this purpose), so the C ABI
@@ -56,8 +57,10 @@ def parse_header(text: str):
 
 _STRUCT_FIELDS, FUNCTIONS = parse_header(HEADER.read_text())
 STRUCTS = {name: type(name, (ctypes.Structure,), {"_fields_": fields}) for name, fields in _STRUCT_FIELDS.items()}
+_FIELD_NAMES = {name: frozenset(f for f, _ in fields) for name, fields in _STRUCT_FIELDS.items()}
 
 _lib = None
+_native = None
 
 
 def lib():
@@ -82,9 +85,24 @@ def lib():
     return _lib
 
 
+def native():
+    """The CPython extension, with the C ABI library it calls loaded and checked."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise RuntimeError(f"quamba_b200/_native.so cannot be loaded ({e}): build it with `python -m quamba_b200.build`") from e
+        from .modules import plain_types
+        mod.set_types(plain_types())
+        _native = mod
+    return _native
+
+
 def make(struct_name: str, **kw):
     st = STRUCTS[struct_name]()
-    names = {f for f, _ in st._fields_}
+    names = _FIELD_NAMES[struct_name]
     for k, v in kw.items():
         if k not in names:
             raise KeyError(f"{struct_name} has no field {k}")
@@ -106,21 +124,31 @@ _trace = None
 def set_call_trace(sink):
     """``sink``: a list to append (fn, start_event, end_event) to, or None to switch tracing off."""
     global _trace
-    _trace = sink
+    _trace = None if sink is None else _Trace(sink)
+    native().set_trace(_trace)
+
+
+class _Trace:
+    def __init__(self, sink):
+        self.sink, self.start = sink, None
+
+    def __call__(self, fn, phase, stream):
+        import torch
+        event = torch.cuda.Event(enable_timing=True)
+        event.record(torch.cuda.ExternalStream(stream))
+        if phase == 0:
+            self.start = event
+        else:
+            self.sink.append((fn, self.start, event))
 
 
 def call(fn: str, args, stream: int):
     f = getattr(lib(), fn)
-    if _trace is None:
-        check(f(ctypes.byref(args), ctypes.c_void_p(stream)))
-        return
-    import torch
-    ext = torch.cuda.ExternalStream(stream)
-    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    e0.record(ext)
+    if _trace is not None:
+        _trace(fn, 0, stream)
     check(f(ctypes.byref(args), ctypes.c_void_p(stream)))
-    e1.record(ext)
-    _trace.append((fn, e0, e1))
+    if _trace is not None:
+        _trace(fn, 1, stream)
 
 
 PATH_SSD_PORTABLE, PATH_HADAMARD_SIMT, PATH_GEMM_SMALL_TILES, PATH_UPDATE_CTA_TILES = 1, 2, 4, 8

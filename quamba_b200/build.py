@@ -1,52 +1,76 @@
-"""Build the CUDA library in-tree with nvcc for sm_100a (no JIT cache, no torch extension).
+"""Builds the two native libraries in-tree (no JIT cache, no torch extension machinery):
 
-    python -m quamba_b200.build            # builds quamba_b200/libquamba_b200.so if out of date
+    libquamba_b200.so   the kernels behind the C ABI, nvcc for sm_100a
+    _native.so          the host path (CPython extension over torch's C++ API), g++
+
+    python -m quamba_b200.build            # rebuilds what is out of date
 """
 import os
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libquamba_b200.so"
+NATIVE = PKG / "_native.so"
 SOURCES = ["lib.cu", "conv1d.cu", "hadamard.cu", "hadamard_tc.cu", "sscan.cu", "ssd.cu", "ssd_tc.cu", "linear.cu", "gemm_tc.cu", "norm.cu",
            "embedding.cu", "decode.cu", "peer.cu"]
+NATIVE_SOURCES = ["binding.cpp", "binding_layers.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v"]
+CUDA = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 
 
 def _stale(obj: Path, src: Path) -> bool:
     if not obj.exists():
         return True
     t = obj.stat().st_mtime
-    deps = [src] + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.inc")) + [PKG.parent / "include" / "quamba_b200.h"]
-    return any(d.stat().st_mtime > t for d in deps)
+    headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.inc")) if src.suffix == ".cu" else list(CSRC.glob("*.h"))
+    return any(d.stat().st_mtime > t for d in [src, PKG.parent / "include" / "quamba_b200.h"] + headers)
+
+
+def _older(target: Path, objs) -> bool:
+    return not target.exists() or any(Path(o).stat().st_mtime > target.stat().st_mtime for o in objs)
+
+
+def _native_flags():
+    import torch
+    inc = Path(torch.__file__).parent / "include"
+    dirs = [inc, inc / "torch" / "csrc" / "api" / "include", CUDA / "include", sysconfig.get_paths()["include"]]
+    return ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[f for d in dirs for f in ("-isystem", str(d))]], Path(torch.__file__).parent / "lib"
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    nvcc = os.environ.get("NVCC", str(CUDA / "bin" / "nvcc"))
+    cxx = os.environ.get("CXX", "g++")
     objdir = PKG / "build"
     objdir.mkdir(exist_ok=True)
-    objs, procs = [], []
-    for name in SOURCES:
+    flags, torch_lib = _native_flags()
+    procs = []
+    for name in SOURCES + NATIVE_SOURCES:
         src, obj = CSRC / name, objdir / (name + ".o")
-        objs.append(obj)
         if force or _stale(obj, src):
-            cmd = [nvcc, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)]
-            procs.append((name, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+            cmd = [nvcc, *NVCC_FLAGS] if src.suffix == ".cu" else [cxx, *flags]
+            procs.append((name, subprocess.Popen([*cmd, "-c", str(src), "-o", str(obj)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for name, p in procs:
         out, _ = p.communicate()
         if verbose or p.returncode != 0:
-            sys.stderr.write(f"--- nvcc {name} ---\n{out}\n")
+            sys.stderr.write(f"--- {name} ---\n{out}\n")
         (objdir / (name + ".log")).write_text(out)
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed; see the log above")
-    if procs or not LIB.exists():
-        cmd = [nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-gencode", "arch=compute_100a,code=sm_100a"]
-        subprocess.run(cmd, check=True)
+        raise RuntimeError("compilation failed; see the log above")
+    kernels, native = ([str(objdir / (n + ".o")) for n in names] for names in (SOURCES, NATIVE_SOURCES))
+    if _older(LIB, kernels):
+        subprocess.run([nvcc, "-shared", "-o", str(LIB), *kernels, "-gencode", "arch=compute_100a,code=sm_100a"], check=True)
+    if _older(NATIVE, native):
+        subprocess.run([cxx, "-shared", "-o", str(NATIVE), *native, f"-L{PKG}", "-l:libquamba_b200.so",
+                        f"-L{torch_lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"],
+                       check=True)
     return LIB
 
 

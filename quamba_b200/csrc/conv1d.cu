@@ -33,6 +33,8 @@ struct ClSegments {
   const int32_t* dim_group_range;
   int nhead_groups, ndim_groups, headdim, x_group_size, d_state;
   int grouped;
+  int8_t* state;               // nullable: the last four inputs of every channel
+  int64_t st_sb, st_sd, st_sw;
 };
 
 // weight bytes (C, W) -> one word whose byte i multiplies window byte i (= x[l-3+i])
@@ -152,6 +154,20 @@ conv1d_channel_last_kernel(const int8_t* __restrict__ in, int64_t in_sb, int64_t
     p += (int64_t)kUnroll * in_sl;
     o += (int64_t)kUnroll * dsl;
   }
+  if (seg.state != nullptr && l1 == seqlen) {   // the last tile's rows are in L2: read them again instead of tracking them above
+    int8_t* st = seg.state + (int64_t)b * seg.st_sb + (int64_t)c0 * seg.st_sd;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int l = seqlen - 4 + i;
+      const uint32_t r = l >= 0 ? ld_act(reinterpret_cast<const uint32_t*>(src + (int64_t)l * in_sl)) : 0u;
+      if (seg.st_sd == 1) {
+        *reinterpret_cast<uint32_t*>(st + (int64_t)i * seg.st_sw) = r;
+      } else {
+#pragma unroll
+        for (int j = 0; j < kCh; ++j) st[(int64_t)j * seg.st_sd + (int64_t)i * seg.st_sw] = (int8_t)(r >> (8 * j));
+      }
+    }
+  }
 }
 
 // Sequence-last layout.  One thread = 16 consecutive time steps of one (b, d) row.
@@ -160,7 +176,8 @@ conv1d_seq_last_kernel(const int8_t* __restrict__ in, int64_t in_sb, int64_t in_
                        int8_t* __restrict__ out, int64_t out_sb, int64_t out_sd,
                        const int8_t* __restrict__ weight, const int8_t* __restrict__ bias,
                        int batch, int dim, int seqlen, int width, float scale_in, float scale_bias,
-                       float scale_out, int silu, int vec_ok) {
+                       float scale_out, int silu, int vec_ok, int8_t* __restrict__ state, int64_t st_sb, int64_t st_sd,
+                       int64_t st_sw) {
   const int nv = (seqlen + kVec - 1) / kVec;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t total = (int64_t)batch * dim * nv;
@@ -193,6 +210,14 @@ conv1d_seq_last_kernel(const int8_t* __restrict__ in, int64_t in_sb, int64_t in_
         t |= byte << (8 * k);
       }
       w[i] = t;
+    }
+  }
+  if (state != nullptr && v == nv - 1) {   // the row's last four inputs, ending at byte (seqlen - l0) of x[l0 ..]
+    int8_t* st = state + (int64_t)b * st_sb + (int64_t)d * st_sd;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int l = seqlen - 4 + i;
+      st[(int64_t)i * st_sw] = l >= 0 ? src[l] : (int8_t)0;
     }
   }
   uint32_t ow[4];
@@ -315,6 +340,11 @@ int pick_tl(int64_t rows_of_vectors, int seqlen) {
   return tl < 8 ? 8 : tl;
 }
 
+// the channel-last kernel writes a unit-channel-stride state four channels (one word) at a time
+bool state_words_ok(const ClSegments& s) {
+  return s.state == nullptr || s.st_sd != 1 || (aligned(s.state, 4) && s.st_sb % 4 == 0 && s.st_sw % 4 == 0);
+}
+
 int launch_channel_last(const int8_t* in, int64_t in_sb, int64_t in_sl, const int8_t* weight, const int8_t* bias,
                         const ClSegments& seg, int batch, int dim, int seqlen, int width, int silu, cudaStream_t stream) {
   const int cv = dim / kCh;
@@ -370,6 +400,8 @@ extern "C" int qb_quamba2_conv1d_fwd(const qb_quamba2_conv1d_fwd_args* a, void* 
   seg.head_group_range = a->head_group_range; seg.dim_group_range = a->dim_group_range;
   seg.nhead_groups = a->nhead_groups; seg.ndim_groups = a->ndim_groups; seg.headdim = a->x_headdim;
   seg.x_group_size = a->x_dim / a->n_groups; seg.d_state = a->d_state; seg.grouped = grouped ? 1 : 0;
+  seg.state = a->conv_state; seg.st_sb = a->state_sb; seg.st_sd = a->state_sd; seg.st_sw = a->state_sw;
+  QB_REQUIRE(state_words_ok(seg), QB_ERR_INVALID_ARG, "quamba2_conv1d_fwd: conv_state with unit channel stride must be 4-byte aligned");
   return launch_channel_last(a->xBC, a->xBC_sb, a->xBC_sl, a->weight, a->bias, seg, a->batch, a->dim, a->seqlen, a->width,
                              a->silu, (cudaStream_t)stream);
 }
@@ -395,6 +427,8 @@ extern "C" int qb_causal_conv1d_fwd(const qb_conv1d_fwd_args* a, void* stream) {
     }
     seg.out_scale_value = a->scale_out;
     seg.end0 = seg.end1 = a->dim;
+    seg.state = a->conv_state; seg.st_sb = a->state_sb; seg.st_sd = a->state_sd; seg.st_sw = a->state_sw;
+    QB_REQUIRE(state_words_ok(seg), QB_ERR_INVALID_ARG, "causal_conv1d_fwd: conv_state with unit channel stride must be 4-byte aligned");
     return launch_channel_last(a->x, a->x_sb, a->x_sl, a->weight, a->bias, seg, a->batch, a->dim, a->seqlen, a->width,
                                a->silu, (cudaStream_t)stream);
   }
@@ -404,7 +438,7 @@ extern "C" int qb_causal_conv1d_fwd(const qb_conv1d_fwd_args* a, void* stream) {
   const int64_t total = (int64_t)a->batch * a->dim * ceil_div(a->seqlen, kVec);
   conv1d_seq_last_kernel<<<(unsigned)ceil_div(total, 128), 128, 0, (cudaStream_t)stream>>>(
       a->x, a->x_sb, a->x_sd, a->out, a->out_sb, a->out_sd, a->weight, a->bias, a->batch, a->dim, a->seqlen, a->width,
-      a->scale_w * a->scale_x, a->scale_b, a->scale_out, a->silu, vec_ok);
+      a->scale_w * a->scale_x, a->scale_b, a->scale_out, a->silu, vec_ok, a->conv_state, a->state_sb, a->state_sd, a->state_sw);
   QB_LAUNCH_OK("conv1d_seq_last_kernel");
   return QB_OK;
 }

@@ -87,7 +87,7 @@ extern "C" int qb_set_sm_budget(int sms) {
 
 extern "C" const char* qb_last_error(void) { return qb::t_error; }
 
-extern "C" int qb_abi_version(void) { return 1; }
+extern "C" int qb_abi_version(void) { return 2; }
 
 extern "C" int64_t qb_sizeof(const char* name) {
   if (name == nullptr) return -1;

@@ -1,14 +1,15 @@
 """Quantized Mamba2 mixers W4A8QMamba2 / W8A8QMamba2 with the reference's constructor arguments, sub-module
 names (``in_proj``, ``conv1d``, ``qchunk_scan``, ``norm``, ``had``, ``out_proj``), ``forward`` / ``step`` /
-``allocate_inference_cache`` (quamba/qMamba2.py:735-1068, :1071-1406).  Every tensor op of ``forward`` and ``step``
-is one of this package's CUDA entry points; what remains here is views (``split`` of in_proj's int8 output) and
-the copy of the last ``d_conv`` inputs into the conv state.
+``allocate_inference_cache`` (quamba/qMamba2.py:735-1068, :1071-1406).  The launch sequence of a layer made of this
+package's own modules is issued by one native call (csrc/binding_layers.cpp); the op-by-op form here serves layers with
+hooks, replaced sub-modules or unusual tensor layouts, and states what the native form does.
 """
 import copy
 
 import torch
 import torch.nn as nn
 
+from . import _lib
 from .modules import (QHadamard, Quamb2Conv1D, Quamba2ChunkScan, W4A8B8O8LinearParallel, W4A8B16O16Linear,
                       W8A8B8O8LinearParallel, W8A8B16O16Linear)
 from .norm import QRMSNormGated
@@ -105,11 +106,25 @@ class _QMamba2(nn.Module):
         q.had = QHadamard(q.d_inner, x_H_scale=act_scales["out_proj:input"].item(), blocks=getattr(o, "had_blocks", 1))
         return q
 
+    def native_layer(self, norm, hidden, residual, residual_in_fp32, inference_params):
+        """[block norm ->] this mixer in one native call: (output, residual), or the output alone when ``norm`` is None;
+        None when the layer has to be walked module by module."""
+        conv_state = ssm_state = None
+        decode = False
+        if inference_params is not None:
+            conv_state, ssm_state = self._get_states_from_cache(inference_params, hidden.shape[0])
+            decode = inference_params.seqlen_offset > 0
+        return _lib.native().mamba2_layer(norm, self, hidden, residual, residual_in_fp32, conv_state, ssm_state, decode)
+
     # ---- prefill (qMamba2.py:920-994) ------------------------------------------------------------------------------
     @torch.no_grad()
     def forward(self, u, seqlen=None, seq_idx=None, cu_seqlens=None, inference_params=None):
         """u int8: (batch, seqlen, d_model), or (batch * seqlen, d_model) with ``seqlen`` given.  Returns fp16 of the
         same shape."""
+        if seqlen is None and cu_seqlens is None:
+            out = self.native_layer(None, u, None, False, inference_params)
+            if out is not None:
+                return out
         seqlen_og = seqlen
         if seqlen is None:
             batch, seqlen, _ = u.shape

@@ -89,9 +89,14 @@ class Block(nn.Module):
         self.mixer = mixer_cls(dim)
 
     def forward(self, hidden_states, residual=None, inference_params=None, **mixer_kwargs):
+        mixer = self.mixer
+        if not mixer_kwargs and hasattr(mixer, "native_layer"):
+            out = mixer.native_layer(self.norm, hidden_states, residual, self.residual_in_fp32, inference_params)
+            if out is not None:
+                return out
         hidden_states, residual = self.norm(hidden_states, residual=residual, prenorm=True,
                                             residual_in_fp32=self.residual_in_fp32)
-        hidden_states = self.mixer(hidden_states, inference_params=inference_params, **mixer_kwargs)
+        hidden_states = mixer(hidden_states, inference_params=inference_params, **mixer_kwargs)
         return hidden_states, residual
 
     def allocate_inference_cache(self, batch_size, max_seqlen, dtype=None, **kwargs):

@@ -1,0 +1,56 @@
+"""The one-call form of a layer (csrc/binding_layers.cpp) against the same layer walked module by module, which a hook on a
+sub-module selects: the same launches on the same data, so outputs and both caches are equal bit for bit."""
+import pytest
+import torch
+
+from quamba_b200 import InferenceParams
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(weights, grouped):
+    from quamba_b200 import calibrate as cal
+    fm = cal.Mamba2LMFloat(d_model=256, n_layer=1, vocab_size=320, seed=5, w4_group_size={"w4": -1, "w4g128": 128, "w8": None}[weights])
+    ids = torch.randint(0, 320, (2, 64), generator=torch.Generator().manual_seed(5))
+    scales = cal.calibrate(fm, [ids])
+    q = cal.quantize_model(fm, scales, w_bits=8 if weights == "w8" else 4).to("cuda")
+    layer = q.backbone.layers[0]
+    if grouped:
+        m, heads = layer.mixer, layer.mixer.nheads
+        hr = torch.tensor([[heads // 2, heads]], dtype=torch.int32, device="cuda")
+        dr = torch.tensor([[[16, 64], [32, 64]]], dtype=torch.int32, device="cuda")
+        xs = m.conv1d.x_out_scales.reshape(1, 1, 1) * torch.tensor([[[0.8, 1.0], [1.1, 1.2]]], device="cuda")
+        for mod in (m.conv1d, m.qchunk_scan):
+            mod.x_head_group_range, mod.x_dim_group_range = hr, dr
+        m.conv1d.x_out_scales, m.qchunk_scan.x_scales = xs, xs
+        m.qchunk_scan.ssm_state_scale = m.qchunk_scan.ssm_state_scale.reshape(1, 1, 1, 1).expand(1, 2, 2, 128).contiguous()
+    return layer
+
+
+def _run(layer, batch, length, decode, with_residual, native):
+    g = torch.Generator(device="cuda").manual_seed(batch * 1000 + length)
+    h = torch.randn(batch, length, 256, device="cuda", generator=g).half()
+    r = torch.randn(batch, length, 256, device="cuda", generator=g) if with_residual else None
+    conv, ssm = layer.allocate_inference_cache(batch, 8)
+    conv.copy_(torch.randint(-100, 100, conv.shape, device="cuda", generator=g))
+    ssm.copy_(torch.randint(-100, 100, ssm.shape, device="cuda", generator=g))
+    params = InferenceParams(max_seqlen=8, max_batch_size=batch, seqlen_offset=int(decode), key_value_memory_dict={0: (conv, ssm)})
+    hook = None if native else layer.mixer.conv1d.register_forward_hook(lambda *a: None)
+    try:
+        if native:
+            taken = layer.mixer.native_layer(layer.norm, h, r, True, InferenceParams(max_seqlen=8, max_batch_size=batch))
+            assert taken is not None, "the layer was not taken by the one-call form"
+        out, res = layer(h, r, inference_params=params)
+    finally:
+        if hook is not None:
+            hook.remove()
+    return out, res, conv, ssm
+
+
+@pytest.mark.parametrize("weights,grouped", [("w4", False), ("w4g128", True), ("w8", False), ("w8", True)])
+@pytest.mark.parametrize("batch,length,decode,with_residual", [(1, 1, False, True), (2, 3, False, False), (1, 4, False, True), (2, 133, False, True),
+                                                               (1, 1, True, True), (3, 1, True, True), (9, 1, True, False)])
+def test_one_call_layer_equals_the_module_walk(weights, grouped, batch, length, decode, with_residual):
+    layer = _layer(weights, grouped)
+    for got, want in zip(_run(layer, batch, length, decode, with_residual, True), _run(layer, batch, length, decode, with_residual, False)):
+        assert got.dtype == want.dtype and torch.equal(got, want)
