@@ -251,6 +251,11 @@ int qb_hadamard_quant(const qb_hadamard_quant_args* a, void* stream);
  * transposed layout the reference returns).  x_states: (B, D, nchunks, N) int8, nchunks =
  * ceil(L / 2048): the state after each 2048-step chunk, quantised with roundf + clamp.
  * All *_scale are device pointers to one float.
+ * channel_last != 0 (dstate 16, one group; no reference counterpart): element (b, d, l) of u / delta / z lies at
+ * b*sb + d + l*sl and element (b, n, l) of Bm / Cm at b*sb + n + l*sl, as the projections write them, so nothing has to be
+ * transposed; x_states may then be null, and final_state (nullable, (B, D, N) int8 contiguous) receives the last state.
+ * workspace (256-byte aligned scratch of qb_sscan_fwd_workspace_bytes() bytes, contents undefined before and after) lets the
+ * channel-last form cut many rows into equal shares; null: it runs them in waves.
  * ------------------------------------------------------------------------------------------ */
 typedef struct {
   const int8_t* u;
@@ -290,8 +295,18 @@ typedef struct {
   int32_t dstate;
   int32_t n_groups;
   int32_t delta_softplus;
+  int32_t channel_last;
+  int64_t u_sl;
+  int64_t delta_sl;
+  int64_t z_sl;
+  int64_t B_sl;
+  int64_t C_sl;
+  int8_t* final_state;
+  void* workspace;
+  int64_t workspace_bytes;
 } qb_sscan_fwd_args;
 int qb_sscan_fwd(const qb_sscan_fwd_args* a, void* stream);
+int64_t qb_sscan_fwd_workspace_bytes(int32_t batch, int32_t dim);
 
 /* ------------------------------------------------------------------------------------------
  * Single-step state update (decode), int8 state updated in place.

@@ -523,7 +523,7 @@ PyMethodDef kMethods[] = {
     {"set_types", set_types, METH_O, nullptr},
     QBN_METHOD(conv1_fwd), QBN_METHOD(conv1_update), QBN_METHOD(conv2_fwd), QBN_METHOD(conv2_update), QBN_METHOD(hadamard),
     QBN_METHOD(sscan_fwd), QBN_METHOD(sscan_update), QBN_METHOD(ssd), QBN_METHOD(w4a8), QBN_METHOD(w8a8_mm), QBN_METHOD(w8a8_mv),
-    QBN_METHOD(norm_fwd), QBN_METHOD(normgated_fwd), QBN_METHOD(mamba2_layer),
+    QBN_METHOD(norm_fwd), QBN_METHOD(normgated_fwd), QBN_METHOD(mamba2_layer), QBN_METHOD(mamba1_layer),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Host path of quamba_b200 (see csrc/binding.cpp).", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -189,5 +189,6 @@ void w4a8_run(PyObject* prep, const W4Dims& w, const int8_t* a, int64_t lda, int
               int64_t ldo, bool int8, bool transpose, cudaStream_t st);
 
 PyObject* mamba2_layer(const Args& a);
+PyObject* mamba1_layer(const Args& a);
 
 }  // namespace qbn

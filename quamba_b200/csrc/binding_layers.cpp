@@ -8,7 +8,7 @@ Types g_types{};
 
 namespace {
 PyObject *g_hooks = nullptr, *g_pre_hooks = nullptr;         // torch's hooks on every module
-PyTypeObject *g_w4_mamba2 = nullptr, *g_w8_mamba2 = nullptr;
+PyTypeObject *g_w4_mamba2 = nullptr, *g_w8_mamba2 = nullptr, *g_w4_mamba1 = nullptr, *g_w8_mamba1 = nullptr;
 }  // namespace
 
 PyObject* set_types(PyObject*, PyObject* dict) {
@@ -24,6 +24,7 @@ PyObject* set_types(PyObject*, PyObject* dict) {
   t.W4A8B8O8LinearParallel = type("W4A8B8O8LinearParallel"); t.W8A8B8O8Linear = type("W8A8B8O8Linear");
   t.W8A8B8O8LinearParallel = type("W8A8B8O8LinearParallel"); t.W8A8B16O16Linear = type("W8A8B16O16Linear");
   g_w4_mamba2 = type("W4A8QMamba2"); g_w8_mamba2 = type("W8A8QMamba2");
+  g_w4_mamba1 = type("W4A8QMamba"); g_w8_mamba1 = type("W8A8QMamba");
   g_hooks = PyDict_GetItemString(dict, "forward_hooks");
   g_pre_hooks = PyDict_GetItemString(dict, "forward_pre_hooks");
   Py_XINCREF(g_hooks);
@@ -176,7 +177,8 @@ struct Lin {
     return q;
   }
 
-  void run(const int8_t* a, int64_t lda, int64_t rows, void* out, int64_t ldo, cudaStream_t st) const {
+  // as_matrix: the matrix form even for one row, with the two scales applied in the order of to_seqlen_last
+  void run(const int8_t* a, int64_t lda, int64_t rows, void* out, int64_t ldo, cudaStream_t st, bool as_matrix = false) const {
     if (w4) {
       PyObject* p = prepared();
       const W4Dims d = w4_dims(p);
@@ -187,7 +189,9 @@ struct Lin {
     qb_w8a8_gemm_args s{};
     s.a = a; s.b = i8(w); s.out = out; s.a_row_stride = lda; s.b_col_stride = w.stride(1); s.out_row_stride = ldo;
     s.m = rows; s.n = n; s.k = k; s.out_dtype = int8 ? 0 : 1;
-    if (rows == 1 && Py_TYPE(m.self) != g_types.W8A8B8O8LinearParallel) {
+    if (as_matrix) {
+      s.a_scale = f32(sb); s.b_scale = f32(sa);
+    } else if (rows == 1 && Py_TYPE(m.self) != g_types.W8A8B8O8LinearParallel) {
       s.use_alpha = 1;
       s.alpha = m.num(QBN_NAME(alpha));
     } else {
@@ -385,6 +389,113 @@ PyObject* mamba2_layer(const Args& a) {
   QBN_CALL(qb_rmsnorm_gated, s, st);
   const Tensor q = dev.empty({rows, d}, at::kChar);
   had.run(g, q, rows, d, st);
+  Tensor out = dev.empty({batch, len, outp.n}, at::kHalf);
+  outp.run(i8(q), d, rows, out.data_ptr(), outp.n, st);
+  out = layer_output(out, batch, len, outp);
+  return has_norm ? wrap_tuple({out, residual}) : wrap(out);
+}
+
+// The Mamba1 counterpart: (norm | None, mixer, hidden, residual | None, residual_in_fp32, conv_state | None, ssm_state | None,
+// decode).  Prefill runs channel-last from in_proj to the scan, so none of the module walk's transposes exist here.
+PyObject* mamba1_layer(const Args& a) {
+  const Mod mx(a.object(1));
+  const bool has_norm = !a.is_none(0), decode = a.flag(7);
+  if (has_norm) {
+    if (Py_TYPE(mx.self) != g_w4_mamba1 && Py_TYPE(mx.self) != g_w8_mamba1) throw NotPlain{};
+    mx.require_plain(nullptr);
+  }
+  if ((g_hooks != nullptr && PyDict_GET_SIZE(g_hooks) != 0) || (g_pre_hooks != nullptr && PyDict_GET_SIZE(g_pre_hooks) != 0)) throw NotPlain{};
+  const Tensor x = a.tensor(2);
+  if (!x.is_cuda() || x.dim() != 3 || !x.is_contiguous() || x.numel() == 0) throw NotPlain{};
+  const int64_t batch = x.size(0), len = x.size(1), dm = x.size(2), rows = batch * len;
+  if (decode && len != 1) throw NotPlain{};
+  const Lin in(mx, QBN_NAME(in_proj)), xp(mx, QBN_NAME(x_proj)), dtp(mx, QBN_NAME(dt_proj)), outp(mx, QBN_NAME(out_proj));
+  const Mod conv = mx.child(QBN_NAME(conv1d), g_types.QCausalConv1D), scan = mx.child(QBN_NAME(selective_scan), g_types.QSScan),
+            had_m = mx.child(QBN_NAME(had), g_types.QHadamard);
+  const int64_t d = mx.integer(QBN_NAME(d_inner)), ds = mx.integer(QBN_NAME(d_state)), rank = mx.integer(QBN_NAME(dt_rank));
+  if (in.k != dm || in.features != 2 * d || xp.k != d || xp.features != rank + 2 * ds || dtp.k != rank || dtp.features != d || dtp.n != d || outp.k != d ||
+      !in.int8 || !xp.int8 || !dtp.int8 || outp.int8 || ds != 16 || d % 16 != 0 || rank % 4 != 0)
+    throw NotPlain{};
+  const Tensor conv_st = a.opt_tensor(5), ssm_st = a.opt_tensor(6);
+  auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
+  const Tensor cw = conv.tensor(QBN_NAME(weight)), cb = conv.opt_tensor(QBN_NAME(bias));
+  if (decode && !conv_st.defined()) throw NotPlain{};
+  if (cw.dim() != 2 || cw.size(0) != d || cw.size(1) != 4 || !cw.is_contiguous() || (cb.defined() && !cb.is_contiguous()) ||
+      (conv_st.defined() && (conv_st.scalar_type() != at::kChar || !is(conv_st, {batch, d, 4}) || ssm_st.scalar_type() != at::kChar ||
+                             !is(ssm_st, {batch, d, ds}) || !ssm_st.is_contiguous() || conv_st.device() != x.device() ||
+                             (conv_st.stride(1) == 1 && (conv_st.stride(0) % 4 != 0 || conv_st.stride(2) % 4 != 0)))))
+    throw NotPlain{};
+  const Tensor A = scan.tensor(QBN_NAME(A_log)), D = scan.opt_tensor(QBN_NAME(D)), bias = scan.opt_tensor(QBN_NAME(dt_bias));
+  const Tensor As = scan.tensor(QBN_NAME(A_scale)), us = scan.tensor(QBN_NAME(u_scale)), dts = scan.tensor(QBN_NAME(dt_scale)), Bs = scan.tensor(QBN_NAME(B_scale)),
+               Cs = scan.tensor(QBN_NAME(C_scale)), zs = scan.tensor(QBN_NAME(z_scale)), ss = scan.tensor(QBN_NAME(ssm_state_scale));
+  const Tensor Ds = scan.tensor(QBN_NAME(D_scale)), bs = scan.tensor(QBN_NAME(dt_bias_scale));
+  for (const Tensor* t : {&As, &us, &dts, &Bs, &Cs, &zs, &ss, &Ds, &bs})
+    if (t->numel() != 1 || t->scalar_type() != at::kFloat || !t->is_cuda()) throw NotPlain{};
+  if (!is(A, {d, ds}) || !A.is_contiguous() || A.scalar_type() != at::kChar || (D.defined() && (D.numel() != d || !D.is_contiguous())) ||
+      (bias.defined() && (bias.numel() != d || !bias.is_contiguous() || bias.scalar_type() != at::kChar)))
+    throw NotPlain{};
+  const Rotation had(had_m);
+  if (had.blocks <= 0 || d % had.blocks != 0) throw NotPlain{};
+
+  const Device dev(x);
+  const cudaStream_t st = dev.stream;
+  Tensor u = x, residual;
+  if (has_norm) {
+    BlockNorm n(a.object(0), x, a.object(3), a.flag(4), rows, dm, dev);
+    u = n.rows;
+    residual = n.residual;
+  } else if (x.scalar_type() != at::kChar) {
+    throw NotPlain{};
+  }
+  const Tensor xz = dev.empty({rows, in.n}, at::kChar), cx = dev.empty({rows, d}, at::kChar), xd = dev.empty({rows, xp.n}, at::kChar),
+               dt = dev.empty({rows, d}, at::kChar), y = dev.empty({rows, d}, at::kHalf), q = dev.empty({rows, d}, at::kChar);
+  in.run(i8(u), dm, rows, xz.data_ptr(), in.n, st, !decode);
+  int8_t* z = i8(xz) + d;
+  auto conv_common = [&](auto& s) {
+    s.x = i8(xz); s.out = i8(cx); s.weight = i8(cw); s.bias = i8(cb); s.batch = batch; s.dim = d; s.width = 4; s.x_sd = 1; s.out_sd = 1; s.silu = 1;
+    s.scale_x = conv.num(QBN_NAME(input_scale)); s.scale_w = conv.num(QBN_NAME(weight_scale)); s.scale_out = conv.num(QBN_NAME(output_scale));
+    s.scale_b = conv.num(QBN_NAME(bias_scale));
+    if (conv_st.defined()) { s.conv_state = i8(conv_st); s.state_sb = conv_st.stride(0); s.state_sd = conv_st.stride(1); s.state_sw = conv_st.stride(2); }
+  };
+  if (decode) {
+    qb_conv1d_update_args s{};
+    conv_common(s);
+    s.x_sb = in.n; s.out_sb = d;
+    QBN_CALL(qb_causal_conv1d_update, s, st);
+  } else {
+    qb_conv1d_fwd_args s{};
+    conv_common(s);
+    s.seqlen = len; s.x_sb = len * in.n; s.x_sl = in.n; s.out_sb = len * d; s.out_sl = d;
+    QBN_CALL(qb_causal_conv1d_fwd, s, st);
+  }
+  xp.run(i8(cx), d, rows, xd.data_ptr(), xp.n, st);
+  dtp.run(i8(xd), xp.n, rows, dt.data_ptr(), d, st, !decode);
+  int8_t *B = i8(xd) + rank, *C = B + ds;
+  if (decode) {
+    qb_sscan_update_args t{};
+    t.state = i8(ssm_st); t.x = i8(cx); t.dt = i8(dt); t.A_log = i8(A); t.Bm = B; t.Cm = C; t.D = i8(D); t.z = z; t.dt_bias = ptr(bias);
+    t.x_scales = f32(us); t.dt_scale = f32(dts); t.A_scale = f32(As); t.state_scale = f32(ss); t.B_scale = f32(Bs); t.C_scale = f32(Cs); t.D_scale = f32(Ds);
+    t.z_scale = f32(zs); t.dt_bias_scale = f32(bs); t.out = y.data_ptr();
+    t.state_sb = d * ds; t.state_sh = d * ds; t.state_sp = ds; t.x_sb = t.x_sh = d; t.dt_sb = t.dt_sh = d; t.dt_sp = 1; t.A_sh = d * ds; t.A_sp = ds; t.A_sn = 1;
+    t.B_sb = t.B_sg = t.C_sb = t.C_sg = xp.n; t.D_sh = d; t.D_sp = 1; t.z_sb = t.z_sh = in.n; t.bias_sh = d; t.bias_sp = 1; t.out_sb = t.out_sh = d;
+    t.batch = batch; t.nheads = 1; t.headdim = d; t.dstate = ds; t.ngroups = 1; t.dt_softplus = scan.flag(QBN_NAME(delta_softplus));
+    QBN_CALL(qb_sscan_update, t, st);
+  } else {
+    qb_sscan_fwd_args t{};
+    t.u = i8(cx); t.delta = i8(dt); t.z = z; t.Bm = B; t.Cm = C; t.A_log = i8(A); t.D = i8(D); t.delta_bias = i8(bias);
+    t.u_scale = f32(us); t.delta_scale = f32(dts); t.z_scale = f32(zs); t.B_scale = f32(Bs); t.C_scale = f32(Cs); t.A_scale = f32(As); t.D_scale = f32(Ds);
+    t.delta_bias_scale = f32(bs); t.ssm_state_scale = f32(ss); t.out = y.data_ptr();
+    t.u_sb = t.delta_sb = len * d; t.u_sl = t.delta_sl = d; t.u_sd = t.delta_sd = t.z_sd = 1; t.z_sb = len * in.n; t.z_sl = in.n;
+    t.B_sb = t.C_sb = len * xp.n; t.B_sl = t.C_sl = xp.n; t.B_sn = t.C_sn = 1;
+    t.batch = batch; t.dim = d; t.seqlen = len; t.dstate = ds; t.n_groups = 1; t.delta_softplus = scan.flag(QBN_NAME(delta_softplus));
+    t.channel_last = 1;
+    t.final_state = ssm_st.defined() ? i8(ssm_st) : nullptr;
+    t.workspace_bytes = qb_sscan_fwd_workspace_bytes(batch, d);
+    const Tensor ws = t.workspace_bytes > 0 ? dev.empty({t.workspace_bytes}, at::kByte) : Tensor();
+    t.workspace = ptr(ws);
+    QBN_CALL(qb_sscan_fwd, t, st);
+  }
+  had.run(y, q, rows, d, st);
   Tensor out = dev.empty({batch, len, outp.n}, at::kHalf);
   outp.run(i8(q), d, rows, out.data_ptr(), outp.n, st);
   out = layer_output(out, batch, len, outp);

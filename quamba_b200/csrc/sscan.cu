@@ -11,6 +11,7 @@
 #include <algorithm>
 #include "common.cuh"
 #include "tc_common.cuh"
+#include "sscan_fwd.cuh"
 
 namespace qb {
 namespace {
@@ -824,7 +825,7 @@ using namespace qb;
 
 extern "C" int qb_sscan_fwd(const qb_sscan_fwd_args* a, void* stream) {
   QB_REQUIRE(a != nullptr, QB_ERR_INVALID_ARG, "sscan_fwd: null args");
-  QB_REQUIRE(a->u && a->delta && a->Bm && a->Cm && a->A_log && a->out && a->x_states, QB_ERR_INVALID_ARG,
+  QB_REQUIRE(a->u && a->delta && a->Bm && a->Cm && a->A_log && a->out && (a->x_states || a->channel_last), QB_ERR_INVALID_ARG,
              "sscan_fwd: null tensor pointer");
   QB_REQUIRE(a->u_scale && a->delta_scale && a->B_scale && a->C_scale && a->A_scale && a->ssm_state_scale,
              QB_ERR_INVALID_ARG, "sscan_fwd: null scale pointer");
@@ -835,6 +836,8 @@ extern "C" int qb_sscan_fwd(const qb_sscan_fwd_args* a, void* stream) {
   QB_REQUIRE(a->batch > 0 && a->dim > 0 && a->seqlen > 0 && a->n_groups > 0, QB_ERR_INVALID_ARG, "sscan_fwd: empty shape");
   QB_REQUIRE(a->dstate <= 256, QB_ERR_INVALID_ARG, "quant_sscan only supports state dimension <= 256");
   QB_REQUIRE(a->dim % a->n_groups == 0, QB_ERR_INVALID_ARG, "sscan_fwd: dim not divisible by n_groups");
+  if (a->channel_last) return run_sscan_channel_last(*a, (cudaStream_t)stream);
+  QB_REQUIRE(a->final_state == nullptr, QB_ERR_INVALID_ARG, "sscan_fwd: final_state is offered by the channel-last form");
   const int kRows = rows_per_cta(a->dstate);
   QB_REQUIRE(a->n_groups == 1 || (a->dim / a->n_groups) % kRows == 0, QB_ERR_UNSUPPORTED,
              "sscan_fwd: channels per group must be a multiple of %d", kRows);
@@ -859,6 +862,8 @@ extern "C" int qb_sscan_fwd(const qb_sscan_fwd_args* a, void* stream) {
   QB_LAUNCH_OK("sscan_fwd_kernel");
   return QB_OK;
 }
+
+extern "C" int64_t qb_sscan_fwd_workspace_bytes(int32_t batch, int32_t dim) { return batch > 0 && dim > 0 ? sscan_workspace_bytes(batch, dim) : -1; }
 
 extern "C" int qb_sscan_update(const qb_sscan_update_args* a, void* stream) {
   QB_REQUIRE(a != nullptr, QB_ERR_INVALID_ARG, "sscan_update: null args");

@@ -12,6 +12,7 @@ import math
 import torch
 import torch.nn as nn
 
+from . import _lib
 from .modules import (QCausalConv1D, QHadamard, QSScan, W4A8B8O8Linear, W4A8B16O16Linear, W8A8B8O8Linear, W8A8B16O16Linear,
                       _FloatStateMixin)
 
@@ -103,10 +104,24 @@ class _QMamba(nn.Module):
         q.out_proj = cls._linear_from(cls._out_cls, o.out_proj, s["out_proj:input"])
         return q.to(dev)
 
+    def native_layer(self, norm, hidden, residual, residual_in_fp32, inference_params):
+        """[block norm ->] this mixer in one native call (csrc/binding_layers.cpp): (output, residual), or the output alone
+        when ``norm`` is None; None when the layer has to be walked module by module."""
+        conv_state = ssm_state = None
+        decode = False
+        if inference_params is not None:
+            conv_state, ssm_state = self._get_states_from_cache(inference_params, hidden.shape[0])
+            decode = inference_params.seqlen_offset > 0
+        return _lib.native().mamba1_layer(norm, self, hidden, residual, residual_in_fp32, conv_state, ssm_state, decode)
+
     @torch.no_grad()
     def forward(self, hidden_states, inference_params=None):
         """hidden_states int8 (B, L, d_model) -> fp16 (B, L, d_model); with ``inference_params`` the caches are filled
-        (prefill) or one token is decoded (seqlen_offset > 0)."""
+        (prefill) or one token is decoded (seqlen_offset > 0).  The native call runs channel-last; the walk below is the
+        sequence-last form of the reference."""
+        out = self.native_layer(None, hidden_states, None, False, inference_params)
+        if out is not None:
+            return out
         batch, seqlen, _ = hidden_states.shape
         conv_state = ssm_state = None
         if inference_params is not None:

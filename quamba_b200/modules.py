@@ -38,11 +38,11 @@ def _dev(device=None):
 def plain_types():
     """What the native layer functions check before they bypass the modules: the classes they know by name, and torch's
     registries of hooks on every module."""
-    from . import mixer, norm
+    from . import mixer, mixer1, norm
     from torch.nn.modules import module as nn_module
     names = {c.__name__: c for c in (QCausalConv1D, Quamb2Conv1D, QSScan, Quamba2ChunkScan, QHadamard, W4A8B16O16Linear, W4A8B8O8Linear,
                                      W4A8B8O8LinearParallel, W8A8B8O8Linear, W8A8B8O8LinearParallel, W8A8B16O16Linear,
-                                     norm.QRMSNorm, norm.QRMSNormGated, mixer.W4A8QMamba2, mixer.W8A8QMamba2)}
+                                     norm.QRMSNorm, norm.QRMSNormGated, mixer.W4A8QMamba2, mixer.W8A8QMamba2, mixer1.W4A8QMamba, mixer1.W8A8QMamba)}
     return dict(names, forward_hooks=nn_module._global_forward_hooks, forward_pre_hooks=nn_module._global_forward_pre_hooks)
 
 
