@@ -3,16 +3,26 @@
 //
 //   C[m, n] = sum_k A[m, k] * W[n, k]      A (M, K) and W (N, K) both K-contiguous int8.
 //
-// One CTA produces one 128 x 128 output tile.  Warp 0 issues the TMA loads (one elected lane),
-// warp 1 owns the TMEM allocation and issues the MMAs (one elected lane), warps 2..5 run the
-// epilogue: tcgen05.ld of the int32 accumulator, scaling, conversion and stores.  Shared memory
-// holds kStages x (A tile 16 KB + W tile 16 KB); two CTAs fit on an SM so that one CTA's epilogue
-// overlaps the other's main loop.  Out-of-range rows / columns / K tails are zero-filled by TMA
-// and masked in the epilogue, so M, N and K need no padding (K and the row pitches only have to be
-// multiples of 16 bytes, the TMA rule).  Every wait is bounded; on expiry the kernel records
-// QB_ERR_TIMEOUT in the device status word, frees its TMEM and returns.
+// One persistent kernel in two forms, both walking tiles of TR rows x bn columns (bn a runtime multiple of 16):
+//   * pair: two CTAs of a cluster share a 256 x bn tile (cta_group::2).  Each holds its 128 rows of A and HALF of the bn rows
+//     of W, so a K step brings (128 + bn / 2) * 32 bytes through a CTA's shared memory where one CTA on its own would bring
+//     (128 + bn) * 32.  Each CTA's producer loads its own halves and counts them on the LEADER's barrier; the leader issues
+//     every MMA, and its commits release the stages and announce the accumulators in both CTAs.  No load is multicast.
+//   * single: one CTA, up to 128 rows: batched decode, where the weights are streamed once and M fills no second CTA.
+// Warp 0 produces (one elected lane), warp 1 owns the TMEM allocation and issues the MMAs (one elected lane), warps 2..9 run
+// the epilogue: two accumulators in tensor memory, so that the epilogue of a tile overlaps the main loop of the next one.
+//
+// What bounds it, as measured at 16384 x 10240 x 2560 (1.92 POP/s before, 3.36 after):
+//   * the epilogue: with one global load per element for its column scale and 16-byte stores scattered over 32 rows, draining
+//     a 128 x 256 tile took 16000 cycles against 10240 of MMAs; see store_piece64;
+//   * the single issuing and producing threads: some 400 cycles of dependent instructions per stage, hence two slabs of K
+//     (eight MMAs) per stage and one 3-D load per operand and stage;
+//   * L2: the tile order keeps a band of A in L2 while W passes by (16384 x 4096 x 8192: 440 -> 329 us);
+//   * then the power cap: at 1.4 GHz under a sustained load the tensor pipe is busy 85 % of the time.
+// Out-of-range rows / columns / K tails are zero-filled by TMA and masked or dropped in the epilogue, so M, N and K need no
+// padding (K and the row pitches only have to be multiples of 16 bytes, the TMA rule).  Every wait is bounded; on expiry the
+// kernel records QB_ERR_TIMEOUT in the device status word, frees its TMEM and returns.
 #include <algorithm>
-#include <cstdlib>
 #include "tc_common.cuh"
 #include "linear_epilogue.cuh"
 
@@ -20,12 +30,12 @@ namespace qb {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 128;  // BK bytes of K per stage = one swizzle atom row
-constexpr int kStages = 3;
-constexpr int kThreads = 192;
-constexpr int kTileBytes = BM * BK;  // 16 KB (A) and BN * BK = 16 KB (W)
-constexpr int kSmemBytes = kStages * 2 * kTileBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-constexpr uint32_t kTmemCols = 128;
+constexpr int BM = 128, BK = 128;   // rows of A per CTA; bytes of K per slab = one swizzle atom row
+constexpr int kMaxBN = 256;         // columns of a tile, and of a TMEM accumulator
+constexpr int kSlabs = 2;           // slabs per stage
+constexpr int kMaxStages = 8;
+constexpr int kThreads = 64 + 256;
+constexpr int kEpiWarps = 8;
 
 using namespace tc;
 
@@ -73,162 +83,122 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&r)[32], int m, int 
   }
 }
 
-// kBN: tile width.  128 for general shapes; 64 for a single row of tiles (M <= 128, weight streaming), where narrower
-// tiles put a CTA on every SM -- 83 CTAs of 128 columns cannot pull the weights of the 2.7B in_proj at HBM speed.
-// a_rows: rows of A that exist (the TMA box of A; the MMA still multiplies 128 rows, the rest of the tile is whatever
-// shared memory held, and those output rows are masked in the epilogue).
-// kARows: rows of A a stage has room for (a multiple of 8; the MMA's 128-row read then runs on into the stages behind it, whose
-// contents only reach masked output rows), kSt: stages.  Few rows of A leave room for a deeper ring: a decode batch of 16
-// streams its weights through eight 12 KB stages instead of three 24 KB ones.
-template <int kBN, int kARows = BM, int kSt = kStages>
-__global__ void __launch_bounds__(kThreads)
-gemm_s8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                       int M, int N, int K, int a_rows, Epilogue ep, int* status, int early) {
-  if (early) grid_dependency_launch();
-  extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment: the swizzle pattern is a function of the shared-memory address bits.
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = smem;
-  constexpr int kWBytes = kBN * BK;
-  constexpr int kABytes = kARows * BK;
-  static_assert(kARows % 8 == 0 && (BM - kARows) * BK <= kSt * kWBytes, "the 128-row read of the last stage must stay inside the ring");
-  uint8_t* sW = smem + kSt * kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSt * (kABytes + kWBytes));
-  uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + kSt;
-  uint64_t* accum_bar = bars + 2 * kSt;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSt + 1);
+// The epilogue of aligned row-major outputs, 64 columns of a warp's 32 rows at a time: scales from shared memory (one read per
+// four columns for the whole warp instead of one cached global load per element), conversion, and the converted piece leaves
+// through a swizzled shared-memory buffer and one TMA store, so that global memory sees whole 64- or 128-byte row pieces; rows
+// and columns outside the matrix are dropped by the store.  The fp32 steps and their order are those of Epilogue::scaled.
+// int8: clamp, then round half to even by adding 1.5 * 2^23, whose low mantissa byte is the two's complement result (the
+// conversion pipe, 16 results a clock, is left to the int32 -> fp32 conversions).
+constexpr int kOutBuf = 32 * 128;        // bytes of a warp's buffer: 32 rows of 64 fp16 or int8
+__device__ __forceinline__ uint32_t round_s8_bits(float v) { return __float_as_uint(fminf(fmaxf(v, -128.0f), 127.0f) + 12582912.0f); }
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * kBN;
-  const int num_kb = (K + BK - 1) / BK;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kSt; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(accum_bar, 1);
-    fence_barrier_init();
-    prefetch_tensormap(&tmap_a);
-    prefetch_tensormap(&tmap_w);
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  // launched as a programmatic dependent: barriers, tensor memory and descriptors above were set up while the kernel
-  // before this one may still have been running; A (and per-row scales) are read from here on, by TMA or past L1
-  grid_dependency_wait();
-
-  if (warp == 0) {
-    if (lane == 0) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int s = kb % kSt;
-        const uint32_t ph = (kb / kSt) & 1;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1, status, QB_ERR_TIMEOUT)) break;
-        mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(a_rows * BK + kWBytes));
-        tma_load_2d(sA + s * kABytes, &tmap_a, &full_bar[s], kb * BK, m0);
-        tma_load_2d(sW + s * kWBytes, &tmap_w, &full_bar[s], kb * BK, n0);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(/*c=s32*/ 2, /*a=s8*/ 1, /*b=s8*/ 1, 0, 0, BM, kBN);
-      // descriptor words of stage 0; a stage / K step is one 32-bit add away (the issuer's instruction count per MMA
-      // decides whether the tensor pipe stays fed)
-      const SmemDesc da0 = make_smem_desc2(smem_u32(sA), 16, 1024, kSwizzle128B);
-      const SmemDesc dw0 = make_smem_desc2(smem_u32(sW), 16, 1024, kSwizzle128B);
-      bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int s = kb % kSt;
-        const uint32_t ph = (kb / kSt) & 1;
-        ok = mbar_wait(&full_bar[s], ph, status, QB_ERR_TIMEOUT);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const SmemDesc da = desc_advance(da0, (uint32_t)s * kABytes);
-        const SmemDesc dw = desc_advance(dw0, (uint32_t)s * kWBytes);
+__device__ __forceinline__ void store_piece64(const uint32_t (&r0)[32], const uint32_t (&r1)[32], const float* scale, float row_scale, bool f16,
+                                              uint8_t* buf, int lane, const CUtensorMap* map, int n0, int m0) {
+  if (lane == 0) bulk_wait_read<0>();    // the piece before has left the buffer
+  __syncwarp();
 #pragma unroll
-        for (int k = 0; k < BK / 32; ++k)
-          umma_i8(tmem_base, desc_advance(da, k * 32), desc_advance(dw, k * 32), idesc, (kb | k) != 0 ? 1u : 0u);
-        umma_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 16) {
+      float v[16];
+#pragma unroll
+      for (int t = 0; t < 16; t += 4) {
+        const float4 cs = *reinterpret_cast<const float4*>(scale + h * 32 + j + t);
+        const float c[4] = {cs.x, cs.y, cs.z, cs.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[t + e] = ((float)(int)(h == 0 ? r0[j + t + e] : r1[j + t + e]) * c[e]) * row_scale;
       }
-      umma_commit(accum_bar);  // accumulator complete (arrives even after an aborted loop)
-    }
-  } else {
-    // Epilogue warps 2..5: warp w may touch TMEM lanes [32 * (w % 4), 32 * (w % 4) + 32).
-    const int q = warp & 3;
-    const bool ok = mbar_wait(accum_bar, 0, status, QB_ERR_TIMEOUT);
-    tc_fence_after_sync();
-    if (ok) {
-      const int m = m0 + q * 32 + lane;
-#pragma unroll 1
-      for (int c = 0; c < kBN; c += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c, r);
-        tmem_ld_wait();
-        store_chunk(r, m, n0 + c, M, N, ep);
+      if (f16) {                         // 128-byte rows: 16-byte piece p of row r sits at p ^ (r & 7)
+        uint4 w[2];
+        __half2* hp = reinterpret_cast<__half2*>(w);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) hp[t] = __floats2half2_rn(v[2 * t], v[2 * t + 1]);
+        const int p = (h * 32 + j) / 8;
+        *reinterpret_cast<uint4*>(buf + lane * 128 + ((p ^ (lane & 7)) << 4)) = w[0];
+        *reinterpret_cast<uint4*>(buf + lane * 128 + (((p + 1) ^ (lane & 7)) << 4)) = w[1];
+      } else {                           // 64-byte rows: piece p of row r sits at p ^ ((r >> 1) & 3)
+        uint32_t w[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const uint32_t lo = __byte_perm(round_s8_bits(v[4 * t]), round_s8_bits(v[4 * t + 1]), 0x0040);
+          const uint32_t hi = __byte_perm(round_s8_bits(v[4 * t + 2]), round_s8_bits(v[4 * t + 3]), 0x0040);
+          w[t] = __byte_perm(lo, hi, 0x5410);
+        }
+        const int p = (h * 32 + j) / 16;
+        *reinterpret_cast<uint4*>(buf + lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem_base, kTmemCols);
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_2d(map, buf, f16 ? n0 * 2 : n0, m0);
+    bulk_commit();
   }
 }
 
-// ---- persistent variant for large problems -------------------------------------------------------------------------------
-// 128 x 256 tiles (one W tile byte feeds twice the MACs of the 128 x 128 kernel, which keeps the MMAs fed from shared
-// memory at tensor speed), four 48 KB stages, one CTA per SM walking tiles round-robin, and two 256-column accumulators in
-// TMEM so that the epilogue of a tile (warps 2..5) overlaps the main loop of the next one.  Tiles are ordered M-fastest:
-// CTAs that run at the same time read the same W tile, which then comes from L2.
-constexpr int PBN = 256;
-constexpr int kPStages = 4;
-constexpr int kPStageBytes = BM * BK + PBN * BK;   // 16 KB of A + 32 KB of W
-constexpr int kPSmemBytes = kPStages * kPStageBytes + 1024 + 256;
-// Eight epilogue warps (two per TMEM lane quarter, 128 columns each): with four, converting and storing a 128 x 256
-// tile took about as long as the main loop of a K = 2560 tile and the MMA issuer waited for its accumulator.
-constexpr int kPThreads = 64 + 256;
+constexpr int kFixedSmem = kEpiWarps * kOutBuf + 2 * kMaxBN * (int)sizeof(float) + 256;   // output buffers, scales, barriers
+constexpr int kSmemLimit = 232448;                                                       // 227 KB
 
-// bn: tile width actually used (a multiple of 16, <= 256; the TMA box of W has bn rows).  The host picks the width whose
-// tile count fills whole rounds of the grid best: at 2048 rows the 2.7B out_proj (N = 2560) is 160 tiles of 256 columns on
-// 148 SMs, two rounds with the second almost empty, or 224 tiles of 192 columns, two rounds of cheaper tiles.  Shared-memory
-// slots and the TMEM accumulators keep their 256-column size.
-__global__ void __launch_bounds__(kPThreads, 1)
-gemm_s8_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                                  int M, int N, int K, int bn, Epilogue ep, int* status, int early) {
+struct TileShape {
+  int bn;            // tile columns
+  int a_rows;        // rows of A a CTA loads (128, or fewer where M is: the MMA's 128-row read then runs on into whatever
+                     // follows, which only reaches output rows that are dropped)
+  int stages, stage_bytes;
+  int band;          // tile rows per band of the tile order
+  int slab_maps;     // 3-D maps (K a multiple of 128), else one 2-D load per slab
+  int tma_out;       // outputs leave by TMA
+};
+
+template <bool kPair>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_o,
+               int M, int N, int K, const TileShape ts, Epilogue ep, int* status, int early) {
   if (early) grid_dependency_launch();
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPStages * kPStageBytes);
-  uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + kPStages;
-  uint64_t* acc_full = bars + 2 * kPStages;       // [2]
-  uint64_t* acc_empty = bars + 2 * kPStages + 2;  // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kPStages + 4);
+  // aligned for the swizzle patterns, and at the same offset in both CTAs: the leader's descriptors and barrier addresses
+  // are used for its peer's shared memory
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* out_buf = smem + ts.stages * ts.stage_bytes;
+  float* scales = reinterpret_cast<float*>(out_buf + kEpiWarps * kOutBuf);   // [2][kMaxBN]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(scales + 2 * kMaxBN);     // (pair: the leader's are used)
+  uint64_t* empty_bar = full_bar + kMaxStages;                               // one set per CTA
+  uint64_t* acc_full = empty_bar + kMaxStages;                               // [2], one set per CTA
+  uint64_t* acc_empty = acc_full + 2;                                        // [2] (pair: the leader's are used)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
+  constexpr int kCtas = kPair ? 2 : 1, kRows = kCtas * BM;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
+  const uint32_t rank = kPair ? cluster_rank() : 0u;
+  const int unit = blockIdx.x / kCtas, units = gridDim.x / kCtas;
+  const int bn = ts.bn, w_rows = bn / kCtas;
+  const int tiles_m = (M + kRows - 1) / kRows, tiles_n = (N + bn - 1) / bn;
   const int tiles = tiles_m * tiles_n;
-  const int num_kb = (K + BK - 1) / BK;
-  const int my_tiles = (int)blockIdx.x < tiles ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+  const int num_kb = (K + kSlabs * BK - 1) / (kSlabs * BK);                  // stages per tile
+  const int my_tiles = unit < tiles ? (tiles - unit + units - 1) / units : 0;
+  // Tile order: bands of tile rows, M-fastest inside a band.  Units that run at the same time read the same W tile, and a
+  // band's rows of A stay in L2 while all of W passes by.
+  auto tile_at = [&](int i, int& m0, int& n0) {
+    const int t = unit + i * units, per_band = ts.band * tiles_n, g = t / per_band, r = t - g * per_band;
+    const int rows = min(ts.band, tiles_m - g * ts.band), tn = r / rows;
+    m0 = (g * ts.band + (r - tn * rows)) * kRows + (int)rank * BM;
+    n0 = tn * bn;
+  };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 1); }
+    for (int s = 0; s < ts.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kCtas); }
     fence_barrier_init();
     prefetch_tensormap(&tmap_a);
     prefetch_tensormap(&tmap_w);
+    if (ts.tma_out) prefetch_tensormap(&tmap_o);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
+    if (kPair) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+    else { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (kPair) cluster_sync();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   // launched as a programmatic dependent: barriers, tensor memory and descriptors above were set up while the kernel
@@ -237,63 +207,96 @@ gemm_s8_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, co
 
   if (warp == 0) {
     if (lane == 0) {
-      int it = 0;  // k-iterations issued so far, over all tiles: the stage ring runs through tile boundaries
-      for (int i = 0; i < my_tiles; ++i) {
-        const int t = blockIdx.x + i * gridDim.x;
-        const int m0 = (t % tiles_m) * BM, n0 = (t / tiles_m) * bn;
-        bool ok = true;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % kPStages;
-          ok = mbar_wait(&empty_bar[s], (uint32_t)(((it / kPStages) & 1) ^ 1), status, QB_ERR_TIMEOUT);
+      const int a_slab = ts.a_rows * BK, w_slab = w_rows * BK;
+      const uint32_t bytes = (uint32_t)(kCtas * kSlabs * (a_slab + w_slab));
+      const uint32_t bar0 = kPair ? map_to_rank(full_bar, 0) : smem_u32(full_bar);
+      int s = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int i = 0; i < my_tiles && ok; ++i) {
+        int m0, n0;
+        tile_at(i, m0, n0);
+        n0 += (int)rank * w_rows;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = mbar_wait_spin(&empty_bar[s], ph, status, QB_ERR_TIMEOUT);
           if (!ok) break;
-          uint8_t* stage = smem + s * kPStageBytes;
-          mbar_arrive_expect_tx(&full_bar[s], (uint32_t)((BM + bn) * BK));
-          tma_load_2d(stage, &tmap_a, &full_bar[s], kb * BK, m0);
-          tma_load_2d(stage + BM * BK, &tmap_w, &full_bar[s], kb * BK, n0);
+          uint8_t* sa = smem + s * ts.stage_bytes;
+          uint8_t* sw = sa + kSlabs * a_slab;
+          const uint32_t bar = bar0 + 8u * (uint32_t)s;
+          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
+          if (ts.slab_maps) {
+            tma_load_3d<kPair>(sa, &tmap_a, bar, 0, m0, kb * kSlabs);
+            tma_load_3d<kPair>(sw, &tmap_w, bar, 0, n0, kb * kSlabs);
+          } else {
+#pragma unroll
+            for (int j = 0; j < kSlabs; ++j) {
+              tma_load_2d<kPair>(sa + j * a_slab, &tmap_a, bar, (kb * kSlabs + j) * BK, m0);
+              tma_load_2d<kPair>(sw + j * w_slab, &tmap_w, bar, (kb * kSlabs + j) * BK, n0);
+            }
+          }
+          if (++s == ts.stages) { s = 0; ph ^= 1; }
         }
-        if (!ok) break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(/*c=s32*/ 2, /*a=s8*/ 1, /*b=s8*/ 1, 0, 0, BM, (uint32_t)bn);
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc = make_idesc(/*c=s32*/ 2, /*a=s8*/ 1, /*b=s8*/ 1, 0, 0, kRows, (uint32_t)bn);
       const SmemDesc da0 = make_smem_desc2(smem_u32(smem), 16, 1024, kSwizzle128B);
-      int it = 0;
+      const uint32_t a_slab = (uint32_t)(ts.a_rows * BK), w_slab = (uint32_t)(w_rows * BK);
+      int s = 0;
+      uint32_t ph = 0;
       bool ok = true;
       for (int i = 0; i < my_tiles && ok; ++i) {
         const int b = i & 1;
-        ok = mbar_wait(&acc_empty[b], (uint32_t)(((i >> 1) & 1) ^ 1), status, QB_ERR_TIMEOUT);  // epilogue has drained it
+        ok = mbar_wait_spin(&acc_empty[b], (uint32_t)(((i >> 1) & 1) ^ 1), status, QB_ERR_TIMEOUT);  // the epilogue has drained it
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t acc = tmem_base + (uint32_t)(b * PBN);
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % kPStages;
-          ok = mbar_wait(&full_bar[s], (uint32_t)((it / kPStages) & 1), status, QB_ERR_TIMEOUT);
+        const uint32_t acc = tmem_base + (uint32_t)(b * kMaxBN);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = mbar_wait_spin(&full_bar[s], ph, status, QB_ERR_TIMEOUT);
           if (!ok) break;
           tc_fence_after_sync();
-          const SmemDesc da = desc_advance(da0, (uint32_t)s * kPStageBytes);
-          const SmemDesc dw = desc_advance(da, BM * BK);
+          const SmemDesc da = desc_advance(da0, (uint32_t)(s * ts.stage_bytes));
+          const SmemDesc dw = desc_advance(da, kSlabs * a_slab);
 #pragma unroll
-          for (int k = 0; k < BK / 32; ++k)
-            umma_i8(acc, desc_advance(da, k * 32), desc_advance(dw, k * 32), idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit(&empty_bar[s]);
+          for (int j = 0; j < kSlabs; ++j) {
+            const SmemDesc daj = desc_advance(da, j * a_slab), dwj = desc_advance(dw, j * w_slab);
+#pragma unroll
+            for (int k = 0; k < BK / 32; ++k) {
+              if (kPair) umma_i8_pair(acc, desc_advance(daj, k * 32), desc_advance(dwj, k * 32), idesc, (kb | j | k) != 0 ? 1u : 0u);
+              else umma_i8(acc, desc_advance(daj, k * 32), desc_advance(dwj, k * 32), idesc, (kb | j | k) != 0 ? 1u : 0u);
+            }
+          }
+          if (kPair) umma_commit_pair(&empty_bar[s]); else umma_commit(&empty_bar[s]);   // frees the stage once read
+          if (++s == ts.stages) { s = 0; ph ^= 1; }
         }
-        umma_commit(&acc_full[b]);
+        if (kPair) umma_commit_pair(&acc_full[b]); else umma_commit(&acc_full[b]);      // (arrives even after an aborted loop)
       }
     }
   } else {
-    const int q = warp & 3;
-    const int half = (warp - 2) >> 2;   // which half of the tile's 32-column chunks
+    // Epilogue warp w may touch TMEM lanes [32 * (w % 4), 32 * (w % 4) + 32); the two warps of a quarter share its columns.
+    const int q = warp & 3, ew = warp - 2;
+    const int half = ew >> 2;
     const bool lead = warp == 2 && lane == 0;
-    const int nchunks = (bn + 31) / 32;
-    const int c_begin = half == 0 ? 0 : ((nchunks + 1) / 2) * 32;
-    const int c_end = half == 0 ? ((nchunks + 1) / 2) * 32 : nchunks * 32;
+    // 64-column pieces; where bn is no multiple of 64 the last one starts at bn - 64 and repeats columns of the one before
+    const int pieces = (bn + 63) / 64;
+    const int p_begin = half == 0 ? 0 : (pieces + 1) / 2, p_end = half == 0 ? (pieces + 1) / 2 : pieces;
+    const uint32_t leader_empty = kPair ? map_to_rank(acc_empty, 0) : 0u;
     for (int i = 0; i < my_tiles; ++i) {
       const int b = i & 1;
-      const int t = blockIdx.x + i * gridDim.x;
-      const int m0 = (t % tiles_m) * BM, n0 = (t / tiles_m) * bn;
+      int m0, n0;
+      tile_at(i, m0, n0);
       const int n_end = min(N, n0 + bn);      // columns past the tile belong to the next one (or to nobody)
-      // one thread polls, the eight warps meet at a named barrier that also carries the outcome
+      const int m = m0 + q * 32 + lane;
+      // the tile's column scales and this lane's row scale, while the accumulator is still being computed
+      float* sc = scales + b * kMaxBN;
+      float row_scale = 0.0f;
+      if (ts.tma_out) {
+        const int c = threadIdx.x - 64;
+        if (c < bn) sc[c] = n0 + c < N ? ep.col_scale[ep.col_per ? n0 + c : 0] : 0.0f;
+        row_scale = ep.row_scale[ep.row_per ? min(m, M - 1) : 0];
+      }
+      // one thread polls, the eight warps meet at a named barrier that also carries the outcome (and publishes the scales)
       uint32_t ok = 1;
       if (lead) ok = mbar_wait(&acc_full[b], (uint32_t)((i >> 1) & 1), status, QB_ERR_TIMEOUT) ? 1u : 0u;
       uint32_t all_ok;
@@ -301,37 +304,38 @@ gemm_s8_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, co
                    : "=r"(all_ok) : "r"(ok) : "memory");
       if (!all_ok) break;
       tc_fence_after_sync();
-      const int m = m0 + q * 32 + lane;
-      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * PBN);
-      bool released = false;
-#pragma unroll 1
-      for (int c = c_begin; c < c_end; c += 64) {
-        uint32_t r0[32], r1[32];
-        const bool two = c + 32 < c_end;
-        tmem_ld_32x32(acc + (uint32_t)c, r0);
-        if (two) tmem_ld_32x32(acc + (uint32_t)c + 32, r1);
-        tmem_ld_wait();
-        if (c + 64 >= c_end) {  // the last columns are in registers: hand the accumulator back before storing them
-          tc_fence_before_sync();
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          if (lead) mbar_arrive(&acc_empty[b]);
-          released = true;
-        }
-        store_chunk(r0, m, n0 + c, M, n_end, ep);
-        if (two) store_chunk(r1, m, n0 + c + 32, M, n_end, ep);
-      }
-      if (!released) {          // a half without chunks (tile narrower than 64 columns) still takes part in the hand-over
+      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kMaxBN);
+      auto release = [&]() {
         tc_fence_before_sync();
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (lead) mbar_arrive(&acc_empty[b]);
+        if (lead) { if (kPair) mbar_arrive_remote(leader_empty + 8u * (uint32_t)b); else mbar_arrive(&acc_empty[b]); }
+      };
+#pragma unroll 1
+      for (int p = p_begin; p < p_end; ++p) {
+        const int c = max(min(p * 64, bn - 64), 0);
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32(acc + (uint32_t)c, r0);
+        tmem_ld_32x32(acc + (uint32_t)c + 32, r1);
+        tmem_ld_wait();
+        if (p + 1 == p_end) release();        // the last columns are in registers: hand the accumulator back before storing them
+        if (n0 + c >= N || m0 + q * 32 >= M) continue;
+        if (ts.tma_out) {
+          store_piece64(r0, r1, sc + c, row_scale, ep.out_kind == kOutF16, out_buf + ew * kOutBuf, lane, &tmap_o, n0 + c, m0 + q * 32);
+        } else {
+          store_chunk(r0, m, n0 + c, M, n_end, ep);
+          store_chunk(r1, m, n0 + c + 32, M, n_end, ep);
+        }
       }
+      if (p_begin == p_end) release();        // a half without pieces still takes part in the hand-over
     }
+    if (ts.tma_out && lane == 0) bulk_wait_all<0>();
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (kPair) cluster_sync();    // no CTA leaves while its peer's loads, commits or MMAs may still touch its shared memory
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 512);
+    if (kPair) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -342,13 +346,14 @@ gemm_s8_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, co
 // What comes out is the tensor pipe's dense int8 rate with shared-memory operands and no epilogue: the denominator of the
 // GEMM rooflines.
 constexpr int kPeakRing = 4;
+constexpr int kPeakBytes = BM * BK + kMaxBN * BK;
 __global__ void __launch_bounds__(128, 1) i8_mma_peak_kernel(int groups, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPeakBytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kPeakRing);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kPStageBytes / 4; i += blockDim.x)
+  for (int i = threadIdx.x; i < kPeakBytes / 4; i += blockDim.x)
     reinterpret_cast<uint32_t*>(smem)[i] = (uint32_t)(i * 2654435761u) ^ (blockIdx.x * 40503u);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPeakRing; ++s) mbar_init(&bars[s], 1);
@@ -364,14 +369,14 @@ __global__ void __launch_bounds__(128, 1) i8_mma_peak_kernel(int groups, int* st
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = make_idesc(2, 1, 1, 0, 0, BM, PBN);
+    constexpr uint32_t idesc = make_idesc(2, 1, 1, 0, 0, BM, kMaxBN);
     const SmemDesc da = make_smem_desc2(smem_u32(smem), 16, 1024, kSwizzle128B);
     const SmemDesc dw = desc_advance(da, BM * BK);
     bool ok = true;
     for (int g = 0; g < groups && ok; ++g) {
       if (g >= kPeakRing) ok = mbar_wait_spin(&bars[g % kPeakRing], (uint32_t)(((g / kPeakRing) - 1) & 1), status, QB_ERR_TIMEOUT);
       if (!ok) break;
-      const uint32_t acc = tmem_base + (uint32_t)((g & 1) * PBN);
+      const uint32_t acc = tmem_base + (uint32_t)((g & 1) * kMaxBN);
 #pragma unroll
       for (int k = 0; k < 4; ++k) umma_i8(acc, desc_advance(da, k * 32), desc_advance(dw, k * 32), idesc, g >= 2 ? 1u : (k ? 1u : 0u));
       umma_commit(&bars[g % kPeakRing]);
@@ -407,7 +412,7 @@ EncodeTiledFn get_encoder() {
 }  // namespace
 
 int encode_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes,
-                      uint32_t box_rows, uint32_t box_cols) {
+                      uint32_t box_rows, uint32_t box_cols, bool swizzle64) {
   EncodeTiledFn enc = get_encoder();
   QB_REQUIRE(enc != nullptr, QB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const cuuint64_t gdim[2] = {cols, rows};
@@ -415,9 +420,23 @@ int encode_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_
   const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), gdim, gstride, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  QB_REQUIRE(r == CUDA_SUCCESS, QB_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return QB_OK;
+}
+
+int encode_tmap_slabs_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t slabs) {
+  EncodeTiledFn enc = get_encoder();
+  QB_REQUIRE(enc != nullptr, QB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const cuuint64_t gdim[3] = {128, rows, cols / 128};
+  const cuuint64_t gstride[2] = {pitch_bytes, 128};
+  const cuuint32_t box[3] = {128, box_rows, slabs};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), gdim, gstride, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  QB_REQUIRE(r == CUDA_SUCCESS, QB_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  QB_REQUIRE(r == CUDA_SUCCESS, QB_ERR_CUDA, "cuTensorMapEncodeTiled (slabs) failed with code %d", (int)r);
   return QB_OK;
 }
 
@@ -442,76 +461,75 @@ int encode_tmap_f16_4d(CUtensorMap* out, const void* base, const uint64_t dims[4
   return encode_tmap_4d(out, true, true, base, dims, strides_bytes, box);
 }
 
+// Tile columns of the pair form: the candidate whose rounds of the grid cost least.  Measured time per stage (two slabs, all
+// SMs busy, 8192 rows): 745 ns at 256 columns, 654 at 192, 618 at 160, 574 at 128, 493 at 64 -- about 430 + 1.2 bn, the issuing
+// threads' share and the operand traffic -- so a wide tile is nearly free and what counts is the number of rounds.  (208
+// columns ran 10 % above that line and are not offered.)
+int pick_pair_bn(int64_t M, int64_t N, int64_t units) {
+  static const int widths[] = {256, 240, 224, 192, 160, 144, 128, 96, 64};
+  int best = 256;
+  int64_t best_cost = INT64_MAX;
+  for (int w : widths) {
+    const int64_t rounds = ceil_div(ceil_div(M, 2 * BM) * ceil_div(N, w), units), cost = rounds * (430 * 5 + 6 * w);
+    if (cost < best_cost) { best_cost = cost; best = w; }
+  }
+  return best;
+}
+// The single form (at most 128 rows): the narrowest multiple of 16 that needs one round of CTAs, so that all of them stream
+// weights at once, and at least 64.
+int pick_single_bn(int64_t N) {
+  const int64_t per_sm = ceil_div(N, sm_count());
+  return (int)std::min<int64_t>(kMaxBN, std::max<int64_t>(64, ceil_div(per_sm, 16) * 16));
+}
+
+template <bool kPair>
+int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int M, int N, int K, int bn, const Epilogue& ep, int* status, cudaStream_t st) {
+  constexpr int kCtas = kPair ? 2 : 1;
+  TileShape ts{};
+  ts.bn = bn;
+  ts.a_rows = M >= BM ? BM : (int)ceil_div(M, 8) * 8;
+  ts.stage_bytes = kSlabs * BK * (ts.a_rows + bn / kCtas);
+  ts.stages = std::min(kMaxStages, (kSmemLimit - kFixedSmem) / ts.stage_bytes);
+  ts.slab_maps = K % BK == 0;
+  const int64_t tiles_m = ceil_div(M, kCtas * BM), tiles = tiles_m * ceil_div(N, bn);
+  // a band of at most 32 MB of A (L2 holds 126 MB, W tiles and outputs pass through it too)
+  ts.band = (int)std::min<int64_t>(tiles_m, std::max<int64_t>(1, (32 << 20) / ((int64_t)kCtas * BM * K)));
+  const int esize = ep.out_kind == kOutF16 ? 2 : 1;
+  ts.tma_out = !ep.transpose && !ep.use_alpha && (ep.out_kind == kOutF16 || ep.out_kind == kOutS8Rne) && aligned(ep.out, 16) &&
+               ep.out_stride * esize % 16 == 0;
+  CUtensorMap ta, tw, to{};
+  int rc;
+  if (ts.slab_maps) {
+    rc = encode_tmap_slabs_u8(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, ts.a_rows, kSlabs);
+    if (rc == QB_OK) rc = encode_tmap_slabs_u8(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)(bn / kCtas), kSlabs);
+  } else {
+    rc = encode_tmap_2d_u8(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, ts.a_rows, BK);
+    if (rc == QB_OK) rc = encode_tmap_2d_u8(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)(bn / kCtas), BK);
+  }
+  if (rc == QB_OK && ts.tma_out)
+    rc = encode_tmap_2d_u8(&to, ep.out, (uint64_t)M, (uint64_t)N * esize, (uint64_t)ep.out_stride * esize, 32, 64 * esize, esize == 1);
+  if (rc != QB_OK) return rc;
+  static PerDeviceOnce attr;
+  if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_kernel<kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+  const unsigned grid = (unsigned)(std::min<int64_t>(tiles, sm_count() / kCtas) * kCtas);
+  const size_t smem = (size_t)ts.stages * ts.stage_bytes + kFixedSmem;
+  const int early = early_overlap() ? 1 : 0;
+  if (kPair) launch_dependent_cluster(gemm_s8_kernel<kPair>, 2, dim3(grid), dim3(kThreads), smem, st, ta, tw, to, M, N, K, ts, ep, status, early);
+  else launch_dependent(gemm_s8_kernel<kPair>, dim3(grid), dim3(kThreads), smem, st, ta, tw, to, M, N, K, ts, ep, status, early);
+  QB_LAUNCH_OK("gemm_s8_kernel");
+  return QB_OK;
+}
+
 int launch_tensor_core_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int M, int N, int K,
                             const Epilogue& ep, cudaStream_t st) {
   // TMA rules: 16-byte aligned bases and pitches; the inner extent must cover whole 16-byte units.
   if (K % 16 != 0 || lda % 16 != 0 || ldw % 16 != 0 || !aligned(A, 16) || !aligned(W, 16)) return QB_ERR_UNSUPPORTED;
   if (M < 9) return QB_ERR_UNSUPPORTED;   // a few rows are weight-streaming work for the dp4a kernel
-  CUtensorMap ta, tw;
-  int rc = encode_tmap_2d_u8(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, BK);
-  if (rc != QB_OK) return rc;
   int* status = device_status_ptr();
   QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "device status word unavailable");
-  static bool attr_set[64] = {};
-  int dev = 0;
-  QB_CUDA_OK(cudaGetDevice(&dev));
-  const bool no_persistent = path_override(QB_PATH_GEMM_SMALL_TILES);
-  const int64_t ptiles = ceil_div(M, BM) * ceil_div(N, PBN);
-  if (!no_persistent && ptiles >= sm_count()) {   // enough 128 x 256 tiles to give every SM at least one
-    // tile width: the one whose rounds of the grid cost least (rounds x width); ties go to the wider tile.  Only multiples
-    // of 64 columns: 144 .. 240 in steps of 16 were measured too, and every width that is not a multiple of 64 ran 25-90 %
-    // slower per column than its neighbours.  128- and 64-column tiles were measured at the 2.7B layer shapes as well (2048
-    // and 8192 rows) and lost everywhere (10-20 % and 60-110 % slower): every column of W a tile does not cover is another
-    // pass of the A tile through shared memory.
-    int bn = PBN;
-    int64_t best = INT64_MAX;
-    for (int cand = PBN; cand >= 192; cand -= 64) {
-      const int64_t t = ceil_div(M, BM) * ceil_div(N, cand);
-      const int64_t cost = ceil_div(t, sm_count()) * cand;
-      if (cost < best) { best = cost; bn = cand; }
-    }
-    rc = encode_tmap_2d_u8(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)bn, BK);
-    if (rc != QB_OK) return rc;
-    static bool pattr_set[64] = {};
-    if (dev >= 64 || !pattr_set[dev]) {
-      QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_tcgen05_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmemBytes));
-      if (dev < 64) pattr_set[dev] = true;
-    }
-    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(M, BM) * ceil_div(N, bn), sm_count());
-    launch_dependent(gemm_s8_tcgen05_persistent_kernel, dim3(grid), dim3(kPThreads), (size_t)kPSmemBytes, st, ta, tw, M, N, K, bn, ep, status,
-                     early_overlap() ? 1 : 0);
-    QB_LAUNCH_OK("gemm_s8_tcgen05_persistent_kernel");
-    return QB_OK;
-  }
-  // a single row of tiles with too few 128-column tiles to occupy the GPU: 64-column tiles, and only the rows of A that exist
-  const bool narrow = M <= BM && ceil_div(N, BN) < sm_count();
-  const int bn = narrow ? 64 : BN;   // (32-column tiles were slower: every CTA re-reads the A tile)
-  const int a_rows = narrow ? (int)std::min<int64_t>(BM, ceil_div(M, 8) * 8) : BM;
-  if (narrow) {
-    rc = encode_tmap_2d_u8(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, a_rows, BK);
-    if (rc != QB_OK) return rc;
-  }
-  rc = encode_tmap_2d_u8(&tw, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, BK);
-  if (rc != QB_OK) return rc;
-  constexpr int kSmem32 = 8 * (32 * BK + 64 * BK) + 1024 + 256;     // <64, 32 rows, 8 stages>
-  constexpr int kSmem64 = 6 * (64 * BK + 64 * BK) + 1024 + 256;     // <64, 64 rows, 6 stages>
-  if (dev >= 64 || !attr_set[dev]) {
-    QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_tcgen05_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_tcgen05_kernel<64, 32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem32));
-    QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_tcgen05_kernel<64, 64, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
-    if (dev < 64) attr_set[dev] = true;
-  }
-  dim3 grid((unsigned)ceil_div(M, BM), (unsigned)ceil_div(N, bn));
-  const int early = early_overlap() ? 1 : 0;
-  if (bn == 64 && a_rows <= 32)
-    launch_dependent(gemm_s8_tcgen05_kernel<64, 32, 8>, grid, dim3(kThreads), (size_t)kSmem32, st, ta, tw, M, N, K, a_rows, ep, status, early);
-  else if (bn == 64 && a_rows <= 64)
-    launch_dependent(gemm_s8_tcgen05_kernel<64, 64, 6>, grid, dim3(kThreads), (size_t)kSmem64, st, ta, tw, M, N, K, a_rows, ep, status, early);
-  else if (bn == 64) launch_dependent(gemm_s8_tcgen05_kernel<64>, grid, dim3(kThreads), (size_t)kSmemBytes, st, ta, tw, M, N, K, a_rows, ep, status, early);
-  else launch_dependent(gemm_s8_tcgen05_kernel<128>, grid, dim3(kThreads), (size_t)kSmemBytes, st, ta, tw, M, N, K, a_rows, ep, status, early);
-  QB_LAUNCH_OK("gemm_s8_tcgen05_kernel");
-  return QB_OK;
+  if (path_override(QB_PATH_GEMM_SMALL_TILES)) return launch_gemm<false>(A, lda, W, ldw, M, N, K, 128, ep, status, st);
+  if (M <= BM || sm_count() < 2) return launch_gemm<false>(A, lda, W, ldw, M, N, K, M <= BM ? pick_single_bn(N) : 256, ep, status, st);
+  return launch_gemm<true>(A, lda, W, ldw, M, N, K, pick_pair_bn(M, N, sm_count() / 2), ep, status, st);
 }
 
 }  // namespace qb
@@ -524,7 +542,7 @@ extern "C" int qb_i8_mma_peak(int groups, int repeats, void* stream, double* top
   int* status = device_status_ptr();
   QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "device status word unavailable");
   static PerDeviceOnce attr;
-  constexpr int smem = kPStageBytes + 1024 + 256;
+  constexpr int smem = kPeakBytes + 1024 + 256;
   if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(i8_mma_peak_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   cudaStream_t st = (cudaStream_t)stream;
   cudaEvent_t e0, e1;
@@ -541,7 +559,7 @@ extern "C" int qb_i8_mma_peak(int groups, int repeats, void* stream, double* top
   QB_CUDA_OK(cudaEventElapsedTime(&t, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  const double ops = 2.0 * BM * PBN * 32 * 4.0 * groups * (double)sms * repeats;
+  const double ops = 2.0 * BM * kMaxBN * 32 * 4.0 * groups * (double)sms * repeats;
   *tops = ops / (t * 1e-3) / 1e12;
   if (ms != nullptr) *ms = t;
   return QB_OK;
