@@ -8,7 +8,10 @@
 //     of W, so a K step brings (128 + bn / 2) * 32 bytes through a CTA's shared memory where one CTA on its own would bring
 //     (128 + bn) * 32.  Each CTA's producer loads its own halves and counts them on the LEADER's barrier; the leader issues
 //     every MMA, and its commits release the stages and announce the accumulators in both CTAs.  No load is multicast.
-//   * single: one CTA, up to 128 rows: batched decode, where the weights are streamed once and M fills no second CTA.
+//   * single: one CTA, up to 128 rows: batched decode, where the weights are streamed once and M fills no second CTA.  Where
+//     the columns alone do not put a CTA on every SM, K is cut over the CTAs of a cluster: each accumulates its share, leaves
+//     the int32 partial tile in its shared memory, and after a cluster barrier finishes a slice of the columns from all of
+//     them (integers: the sum is the same in any order).
 // Warp 0 produces (one elected lane), warp 1 owns the TMEM allocation and issues the MMAs (one elected lane), warps 2..9 run
 // the epilogue: two accumulators in tensor memory, so that the epilogue of a tile overlaps the main loop of the next one.
 //
@@ -144,11 +147,18 @@ struct TileShape {
   int bn;            // tile columns
   int a_rows;        // rows of A a CTA loads (128, or fewer where M is: the MMA's 128-row read then runs on into whatever
                      // follows, which only reaches output rows that are dropped)
-  int stages, stage_bytes;
+  int stages, stage_bytes, ring_bytes;
   int band;          // tile rows per band of the tile order
+  int splits;        // single form: CTAs of a cluster that share one tile's K
   int slab_maps;     // 3-D maps (K a multiple of 128), else one 2-D load per slab
   int tma_out;       // outputs leave by TMA
 };
+
+__device__ __forceinline__ int4 ld_cluster_int4(uint32_t addr) {
+  int4 v;
+  asm volatile("ld.shared::cluster.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 
 template <bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -158,7 +168,7 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   // aligned for the swizzle patterns, and at the same offset in both CTAs: the leader's descriptors and barrier addresses
   // are used for its peer's shared memory
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* out_buf = smem + ts.stages * ts.stage_bytes;
+  uint8_t* out_buf = smem + ts.ring_bytes;
   float* scales = reinterpret_cast<float*>(out_buf + kEpiWarps * kOutBuf);   // [2][kMaxBN]
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(scales + 2 * kMaxBN);     // (pair: the leader's are used)
   uint64_t* empty_bar = full_bar + kMaxStages;                               // one set per CTA
@@ -169,11 +179,14 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   constexpr int kCtas = kPair ? 2 : 1, kRows = kCtas * BM;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = kPair ? cluster_rank() : 0u;
-  const int unit = blockIdx.x / kCtas, units = gridDim.x / kCtas;
+  const int group = kPair ? 2 : ts.splits;                                   // CTAs of a cluster
+  const int unit = blockIdx.x / group, units = gridDim.x / group;
+  const int split = !kPair && ts.splits > 1 ? (int)cluster_rank() : 0;
   const int bn = ts.bn, w_rows = bn / kCtas;
   const int tiles_m = (M + kRows - 1) / kRows, tiles_n = (N + bn - 1) / bn;
   const int tiles = tiles_m * tiles_n;
-  const int num_kb = (K + kSlabs * BK - 1) / (kSlabs * BK);                  // stages per tile
+  const int all_kb = (K + kSlabs * BK - 1) / (kSlabs * BK);                  // stages per tile
+  const int kb_begin = split * all_kb / ts.splits, num_kb = (split + 1) * all_kb / ts.splits - kb_begin;
   const int my_tiles = unit < tiles ? (tiles - unit + units - 1) / units : 0;
   // Tile order: bands of tile rows, M-fastest inside a band.  Units that run at the same time read the same W tile, and a
   // band's rows of A stay in L2 while all of W passes by.
@@ -224,14 +237,15 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           uint8_t* sw = sa + kSlabs * a_slab;
           const uint32_t bar = bar0 + 8u * (uint32_t)s;
           if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
+          const int k0 = (kb_begin + kb) * kSlabs;
           if (ts.slab_maps) {
-            tma_load_3d<kPair>(sa, &tmap_a, bar, 0, m0, kb * kSlabs);
-            tma_load_3d<kPair>(sw, &tmap_w, bar, 0, n0, kb * kSlabs);
+            tma_load_3d<kPair>(sa, &tmap_a, bar, 0, m0, k0);
+            tma_load_3d<kPair>(sw, &tmap_w, bar, 0, n0, k0);
           } else {
 #pragma unroll
             for (int j = 0; j < kSlabs; ++j) {
-              tma_load_2d<kPair>(sa + j * a_slab, &tmap_a, bar, (kb * kSlabs + j) * BK, m0);
-              tma_load_2d<kPair>(sw + j * w_slab, &tmap_w, bar, (kb * kSlabs + j) * BK, n0);
+              tma_load_2d<kPair>(sa + j * a_slab, &tmap_a, bar, (k0 + j) * BK, m0);
+              tma_load_2d<kPair>(sw + j * w_slab, &tmap_w, bar, (k0 + j) * BK, n0);
             }
           }
           if (++s == ts.stages) { s = 0; ph ^= 1; }
@@ -281,6 +295,7 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // 64-column pieces; where bn is no multiple of 64 the last one starts at bn - 64 and repeats columns of the one before
     const int pieces = (bn + 63) / 64;
     const int p_begin = half == 0 ? 0 : (pieces + 1) / 2, p_end = half == 0 ? (pieces + 1) / 2 : pieces;
+    const int part_pitch = bn * 4 + 16;       // conflict-free 16-byte accesses by 32 rows
     const uint32_t leader_empty = kPair ? map_to_rank(acc_empty, 0) : 0u;
     for (int i = 0; i < my_tiles; ++i) {
       const int b = i & 1;
@@ -291,7 +306,7 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // the tile's column scales and this lane's row scale, while the accumulator is still being computed
       float* sc = scales + b * kMaxBN;
       float row_scale = 0.0f;
-      if (ts.tma_out) {
+      if (ts.tma_out || ts.splits > 1) {
         const int c = threadIdx.x - 64;
         if (c < bn) sc[c] = n0 + c < N ? ep.col_scale[ep.col_per ? n0 + c : 0] : 0.0f;
         row_scale = ep.row_scale[ep.row_per ? min(m, M - 1) : 0];
@@ -319,7 +334,16 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         tmem_ld_wait();
         if (p + 1 == p_end) release();        // the last columns are in registers: hand the accumulator back before storing them
         if (n0 + c >= N || m0 + q * 32 >= M) continue;
-        if (ts.tma_out) {
+        if (!kPair && ts.splits > 1) {        // the partial tile, in the stages (every MMA that read them has completed)
+          int4* dst = reinterpret_cast<int4*>(smem + (q * 32 + lane) * part_pitch + c * 4);
+          if (m < M) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              dst[j] = make_int4(r0[4 * j], r0[4 * j + 1], r0[4 * j + 2], r0[4 * j + 3]);
+              dst[8 + j] = make_int4(r1[4 * j], r1[4 * j + 1], r1[4 * j + 2], r1[4 * j + 3]);
+            }
+          }
+        } else if (ts.tma_out) {
           store_piece64(r0, r1, sc + c, row_scale, ep.out_kind == kOutF16, out_buf + ew * kOutBuf, lane, &tmap_o, n0 + c, m0 + q * 32);
         } else {
           store_chunk(r0, m, n0 + c, M, n_end, ep);
@@ -330,9 +354,52 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
     if (ts.tma_out && lane == 0) bulk_wait_all<0>();
   }
+  if (!kPair && ts.splits > 1) {
+    cluster_sync();                           // all partial tiles are in shared memory
+    int m0, n0;
+    tile_at(0, m0, n0);
+    const int quads = bn / 4, q_begin = split * quads / ts.splits, q_count = (split + 1) * quads / ts.splits - q_begin;
+    const uint32_t base = smem_u32(smem), pitch = (uint32_t)(bn * 4 + 16);
+    const bool vec = !ep.transpose && ep.out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(ep.out) & 7) == 0 && N % 4 == 0 &&
+                     (ep.out_kind == kOutF16 || ep.out_kind == kOutS8Rne) && !ep.use_alpha;
+    for (int i = threadIdx.x; i < M * q_count; i += kThreads) {
+      const int m = i / q_count, c = (q_begin + i % q_count) * 4;
+      const uint32_t addr = base + (uint32_t)m * pitch + (uint32_t)c * 4;
+      int4 v[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {           // all shares of a quad are in flight together
+        if (r < ts.splits) {
+          uint32_t ra;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(r));
+          v[r] = ld_cluster_int4(ra);
+        }
+      }
+      int a4[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (r < ts.splits) { a4[0] += v[r].x; a4[1] += v[r].y; a4[2] += v[r].z; a4[3] += v[r].w; }
+      if (vec && n0 + c < N) {
+        const float rs = ep.row_scale[ep.row_per ? m : 0];
+        float f[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f[e] = ((float)a4[e] * scales[c + e]) * rs;
+        const int64_t at = (int64_t)m * ep.out_stride + n0 + c;
+        if (ep.out_kind == kOutF16) {
+          __half2 h[2] = {__floats2half2_rn(f[0], f[1]), __floats2half2_rn(f[2], f[3])};
+          *reinterpret_cast<uint2*>(static_cast<__half*>(ep.out) + at) = *reinterpret_cast<const uint2*>(h);
+        } else {
+          *reinterpret_cast<uint32_t*>(static_cast<int8_t*>(ep.out) + at) = pack4_s8(rint_s8(f[0]), rint_s8(f[1]), rint_s8(f[2]), rint_s8(f[3]));
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (n0 + c + e < N) ep.store(a4[e], m, n0 + c + e);
+      }
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
-  if (kPair) cluster_sync();    // no CTA leaves while its peer's loads, commits or MMAs may still touch its shared memory
+  if (kPair || ts.splits > 1) cluster_sync();    // no CTA leaves while its peer's loads, commits or MMAs may still touch its shared memory
   if (warp == 1) {
     tc_fence_after_sync();
     if (kPair) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);
@@ -475,18 +542,33 @@ int pick_pair_bn(int64_t M, int64_t N, int64_t units) {
   }
   return best;
 }
-// The single form (at most 128 rows): the narrowest multiple of 16 that needs one round of CTAs, so that all of them stream
-// weights at once, and at least 64.
-int pick_single_bn(int64_t N) {
-  const int64_t per_sm = ceil_div(N, sm_count());
-  return (int)std::min<int64_t>(kMaxBN, std::max<int64_t>(64, ceil_div(per_sm, 16) * 16));
+// The single form (at most 128 rows).  Without a split: the narrowest multiple of 16 (and at least 64) columns that needs one
+// round of CTAs, so that all of them stream weights at once.  Where that leaves SMs idle, K is split over clusters of two, four
+// or eight: what a CTA takes is its stages times what a stage brings, plus about two stages' worth for the exchange.
+// (16 rows, 5120 -> 2560: 40 CTAs of 20 stages, 11.7 us; 128 CTAs of 2 to 3 stages, 6 us.)
+struct SingleShape { int bn, splits; };
+int cluster_capacity(int splits);            // CTAs of clusters of `splits` that are resident at once
+SingleShape pick_single(int64_t N, int64_t K, int a_rows) {
+  const int64_t stages = ceil_div(K, kSlabs * BK);
+  SingleShape best{(int)std::min<int64_t>(kMaxBN, std::max<int64_t>(64, ceil_div(ceil_div(N, sm_count()), 16) * 16)), 1};
+  int64_t best_cost = stages * (best.bn + a_rows + 64);
+  if (ceil_div(N, 64) * 2 > sm_count()) return best;      // the columns alone occupy half the SMs: the exchange costs more than it gives
+  for (int splits = 2; splits <= 8 && splits <= stages; splits *= 2)
+    for (int bn = 64; bn <= kMaxBN; bn += 16) {
+      if (ceil_div(N, bn) * splits > cluster_capacity(splits)) continue;
+      const int64_t cost = (ceil_div(stages, splits) + 2) * (bn + a_rows + 64);
+      if (cost < best_cost) { best_cost = cost; best = SingleShape{bn, splits}; }
+    }
+  return best;
 }
 
 template <bool kPair>
-int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int M, int N, int K, int bn, const Epilogue& ep, int* status, cudaStream_t st) {
+int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int M, int N, int K, int bn, int splits, const Epilogue& ep, int* status,
+                cudaStream_t st) {
   constexpr int kCtas = kPair ? 2 : 1;
   TileShape ts{};
   ts.bn = bn;
+  ts.splits = splits;
   ts.a_rows = M >= BM ? BM : (int)ceil_div(M, 8) * 8;
   ts.stage_bytes = kSlabs * BK * (ts.a_rows + bn / kCtas);
   ts.stages = std::min(kMaxStages, (kSmemLimit - kFixedSmem) / ts.stage_bytes);
@@ -495,7 +577,7 @@ int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int 
   // a band of at most 32 MB of A (L2 holds 126 MB, W tiles and outputs pass through it too)
   ts.band = (int)std::min<int64_t>(tiles_m, std::max<int64_t>(1, (32 << 20) / ((int64_t)kCtas * BM * K)));
   const int esize = ep.out_kind == kOutF16 ? 2 : 1;
-  ts.tma_out = !ep.transpose && !ep.use_alpha && (ep.out_kind == kOutF16 || ep.out_kind == kOutS8Rne) && aligned(ep.out, 16) &&
+  ts.tma_out = splits == 1 && !ep.transpose && !ep.use_alpha && (ep.out_kind == kOutF16 || ep.out_kind == kOutS8Rne) && aligned(ep.out, 16) &&
                ep.out_stride * esize % 16 == 0;
   CUtensorMap ta, tw, to{};
   int rc;
@@ -509,15 +591,48 @@ int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int 
   if (rc == QB_OK && ts.tma_out)
     rc = encode_tmap_2d_u8(&to, ep.out, (uint64_t)M, (uint64_t)N * esize, (uint64_t)ep.out_stride * esize, 32, 64 * esize, esize == 1);
   if (rc != QB_OK) return rc;
+  // the stages also hold the partial tile of a split
+  const size_t ring = std::max<size_t>((size_t)ts.stages * ts.stage_bytes, splits > 1 ? (size_t)ts.a_rows * (bn * 4 + 16) : 0);
+  ts.ring_bytes = (int)ceil_div((int64_t)ring, 1024) * 1024;
   static PerDeviceOnce attr;
   if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_kernel<kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
-  const unsigned grid = (unsigned)(std::min<int64_t>(tiles, sm_count() / kCtas) * kCtas);
-  const size_t smem = (size_t)ts.stages * ts.stage_bytes + kFixedSmem;
+  const size_t smem = (size_t)ts.ring_bytes + kFixedSmem;
+  const int group = kPair ? 2 : splits;
+  const unsigned grid = (unsigned)(std::min<int64_t>(tiles, sm_count() / group) * group);
   const int early = early_overlap() ? 1 : 0;
-  if (kPair) launch_dependent_cluster(gemm_s8_kernel<kPair>, 2, dim3(grid), dim3(kThreads), smem, st, ta, tw, to, M, N, K, ts, ep, status, early);
-  else launch_dependent(gemm_s8_kernel<kPair>, dim3(grid), dim3(kThreads), smem, st, ta, tw, to, M, N, K, ts, ep, status, early);
+  if (group > 1)
+    launch_dependent_cluster(gemm_s8_kernel<kPair>, (unsigned)group, dim3(grid), dim3(kThreads), smem, st, ta, tw, to, M, N, K, ts, ep, status, early);
+  else
+    launch_dependent(gemm_s8_kernel<kPair>, dim3(grid), dim3(kThreads), smem, st, ta, tw, to, M, N, K, ts, ep, status, early);
   QB_LAUNCH_OK("gemm_s8_kernel");
   return QB_OK;
+}
+
+int cluster_capacity(int splits) {
+  static int cached[64][9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+  int& c = cached[dev][splits];
+  if (c == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)splits * 64);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemLimit;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(gemm_s8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_s8_kernel<false>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+    c = n > 0 ? n * splits : -1;
+  }
+  return std::min(c, sm_count());
 }
 
 int launch_tensor_core_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int M, int N, int K,
@@ -527,9 +642,13 @@ int launch_tensor_core_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64
   if (M < 9) return QB_ERR_UNSUPPORTED;   // a few rows are weight-streaming work for the dp4a kernel
   int* status = device_status_ptr();
   QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "device status word unavailable");
-  if (path_override(QB_PATH_GEMM_SMALL_TILES)) return launch_gemm<false>(A, lda, W, ldw, M, N, K, 128, ep, status, st);
-  if (M <= BM || sm_count() < 2) return launch_gemm<false>(A, lda, W, ldw, M, N, K, M <= BM ? pick_single_bn(N) : 256, ep, status, st);
-  return launch_gemm<true>(A, lda, W, ldw, M, N, K, pick_pair_bn(M, N, sm_count() / 2), ep, status, st);
+  if (path_override(QB_PATH_GEMM_SMALL_TILES)) return launch_gemm<false>(A, lda, W, ldw, M, N, K, 128, 1, ep, status, st);
+  if (M <= BM) {
+    const SingleShape s = pick_single(N, K, (int)ceil_div(M, 8) * 8);
+    return launch_gemm<false>(A, lda, W, ldw, M, N, K, s.bn, s.splits, ep, status, st);
+  }
+  if (sm_count() < 2) return launch_gemm<false>(A, lda, W, ldw, M, N, K, kMaxBN, 1, ep, status, st);
+  return launch_gemm<true>(A, lda, W, ldw, M, N, K, pick_pair_bn(M, N, sm_count() / 2), 1, ep, status, st);
 }
 
 }  // namespace qb
