@@ -195,6 +195,34 @@ __device__ __forceinline__ uint32_t pack4_sat_s8(int a, int b, int c, int d) {
   return r;
 }
 
+// Packed fp32 pairs (fma.rn.f32x2 and friends): one issue slot for two operations, each rounded like its scalar form.
+typedef unsigned long long f2;    // two packed floats
+
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// byte k of a word of biased bytes (v + 128) as a float: the byte under the exponent of 2^23
+__device__ __forceinline__ float biased_s8f_raw(uint32_t biased, int k) { return __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7650 + k)); }
+
 // Grouped ("group_heads") lookup: number of cumulative range ends <= idx, clamped to n-1.
 __device__ __forceinline__ int group_lookup(const int32_t* range, int n, int idx) {
   int g = 0;
