@@ -613,7 +613,8 @@ unsigned grid_for(int n, int ctas_per_sm, int nw) {
 template <typename K>
 int opt_in_smem(K kernel, size_t bytes) {
   // per device and per kernel: the attribute is set on every launch that needs it (a cheap host-side call)
-  if (bytes > 48 * 1024) QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  // (below the 48 KB that need no attribute by more than the kernels' own static shared memory)
+  if (bytes > 46 * 1024) QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   return QB_OK;
 }
 
