@@ -306,7 +306,7 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       // the tile's column scales and this lane's row scale, while the accumulator is still being computed
       float* sc = scales + b * kMaxBN;
       float row_scale = 0.0f;
-      if (ts.tma_out || ts.splits > 1) {
+      if (ts.tma_out || (ts.splits > 1 && !ep.use_alpha)) {   // (with the scalar by value there are no scale pointers)
         const int c = threadIdx.x - 64;
         if (c < bn) sc[c] = n0 + c < N ? ep.col_scale[ep.col_per ? n0 + c : 0] : 0.0f;
         row_scale = ep.row_scale[ep.row_per ? min(m, M - 1) : 0];
