@@ -38,13 +38,16 @@ int qb_abi_version(void);
 /* sizeof() of an argument struct by name, for binding self-checks; -1 if unknown. */
 int64_t qb_sizeof(const char* struct_name);
 /* Cross-check switches: a bit set here sends the op to its portable twin (the five-stage SSD path, the SIMT Hadamard
- * kernel, the 128 x 128 GEMM kernel, the CTA-tile state update) so that two implementations can be compared on one
+ * kernel, one-CTA 128 x 128 tiles of the GEMM, the CTA-tile state update) so that two implementations can be compared on one
  * device.  Process-wide, off by default, never read from the environment.  Returns the previous mask. */
 #define QB_PATH_SSD_PORTABLE 1
 #define QB_PATH_HADAMARD_SIMT 2
 #define QB_PATH_GEMM_SMALL_TILES 4
 #define QB_PATH_UPDATE_CTA_TILES 8
 int qb_set_path_override(int mask);
+/* The tile on which the tensor-core GEMM computes an (m, k) x (k, n) product, m > 8, on the current device: its rows (128: one
+ * CTA, 256: a CTA pair), its columns, and the CTAs that share its K.  Tests use it to state which form a size reaches. */
+int qb_gemm_tile(int32_t m, int32_t n, int32_t k, int32_t* rows, int32_t* cols, int32_t* splits);
 /* Caps the number of multiprocessors the library's kernels size their grids for (persistent kernels launch one CTA per
  * SM of the budget; one-wave grids are cut for it).  0 (default) = all SMs of the device.  A caller that overlaps these
  * kernels with a collective on another stream leaves the collective's CTAs room this way: a persistent grid that fills

@@ -3,7 +3,8 @@
 //
 //   C[m, n] = sum_k A[m, k] * W[n, k]      A (M, K) and W (N, K) both K-contiguous int8.
 //
-// One persistent kernel in two forms, both walking tiles of TR rows x bn columns (bn a runtime multiple of 16):
+// One persistent kernel in two forms, both walking tiles of TR rows x bn columns (bn a runtime value: a multiple of 16 for the
+// one-CTA instruction, of 32 for the pair's, the shapes kind::i8 is defined for):
 //   * pair: two CTAs of a cluster share a 256 x bn tile (cta_group::2).  Each holds its 128 rows of A and HALF of the bn rows
 //     of W, so a K step brings (128 + bn / 2) * 32 bytes through a CTA's shared memory where one CTA on its own would bring
 //     (128 + bn) * 32.  Each CTA's producer loads its own halves and counts them on the LEADER's barrier; the leader issues
@@ -528,12 +529,11 @@ int encode_tmap_f16_4d(CUtensorMap* out, const void* base, const uint64_t dims[4
   return encode_tmap_4d(out, true, true, base, dims, strides_bytes, box);
 }
 
-// Tile columns of the pair form: the candidate whose rounds of the grid cost least.  Measured time per stage (two slabs, all
+// Tile columns of the pair form: the multiple of 32 whose rounds of the grid cost least.  Measured time per stage (two slabs, all
 // SMs busy, 8192 rows): 745 ns at 256 columns, 654 at 192, 618 at 160, 574 at 128, 493 at 64 -- about 430 + 1.2 bn, the issuing
-// threads' share and the operand traffic -- so a wide tile is nearly free and what counts is the number of rounds.  (208
-// columns ran 10 % above that line and are not offered.)
+// threads' share and the operand traffic -- so a wide tile is nearly free and what counts is the number of rounds.
 int pick_pair_bn(int64_t M, int64_t N, int64_t units) {
-  static const int widths[] = {256, 240, 224, 192, 160, 144, 128, 96, 64};
+  static const int widths[] = {256, 224, 192, 160, 128, 96, 64};
   int best = 256;
   int64_t best_cost = INT64_MAX;
   for (int w : widths) {
@@ -566,6 +566,7 @@ template <bool kPair>
 int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int M, int N, int K, int bn, int splits, const Epilogue& ep, int* status,
                 cudaStream_t st) {
   constexpr int kCtas = kPair ? 2 : 1;
+  QB_REQUIRE(bn % (16 * kCtas) == 0 && bn <= kMaxBN, QB_ERR_UNSUPPORTED, "int8 GEMM: no MMA of %d columns", bn);
   TileShape ts{};
   ts.bn = bn;
   ts.splits = splits;
@@ -652,6 +653,17 @@ int launch_tensor_core_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64
 }
 
 }  // namespace qb
+
+extern "C" int qb_gemm_tile(int32_t m, int32_t n, int32_t k, int32_t* rows, int32_t* cols, int32_t* splits) {
+  using namespace qb;
+  QB_REQUIRE(m > 8 && n > 0 && k > 0 && rows && cols && splits, QB_ERR_INVALID_ARG, "gemm_tile: bad arguments");
+  QB_REQUIRE(sm_count() > 1, QB_ERR_CUDA, "gemm_tile: no device");
+  const SingleShape s = m <= BM ? pick_single(n, k, (int)ceil_div(m, 8) * 8) : SingleShape{pick_pair_bn(m, n, sm_count() / 2), 1};
+  *rows = m <= BM ? BM : 2 * BM;
+  *cols = s.bn;
+  *splits = s.splits;
+  return QB_OK;
+}
 
 // Measures the dense int8 tensor rate of the current device (see i8_mma_peak_kernel): runs `repeats` launches of `groups`
 // MMA groups per SM on `stream`, times them with CUDA events and returns TOP/s in *tops.  Blocks the host.

@@ -29,3 +29,20 @@ def test_scalar_by_value_with_k_split(m, dtype):
     c = torch.empty((m, n), dtype=dtype, device="cuda")
     ops.quant_linear_cuda.cutlass_scaled_mv_dq(c, w, a, alpha, 0.0)
     assert torch.equal(c, _convert(torch.tensor(alpha, device="cuda") * acc, dtype))
+
+
+def _tile(m, n, k):
+    import ctypes
+    from quamba_b200 import _lib
+    out = [ctypes.c_int32() for _ in range(3)]
+    _lib.check(_lib.lib().qb_gemm_tile(m, n, k, *map(ctypes.byref, out)))
+    return tuple(v.value for v in out)                            # rows, columns, splits
+
+
+def test_tile_columns_are_mma_shapes():
+    """The int8 MMA of a CTA pair takes multiples of 32 columns, that of one CTA multiples of 16; both up to 256."""
+    for m in (9, 16, 65, 128, 129, 300, 512, 777, 1024, 2048, 3000, 4096, 8192, 16384):
+        for n in (16, 64, 192, 320, 768, 1536, 2560, 3024, 4096, 5120, 8192, 8512, 10240, 10576, 18560, 50288):
+            rows, cols, splits = _tile(m, n, 2560)
+            assert 64 <= cols <= 256 and cols % (16 if rows == 128 else 32) == 0, (m, n, rows, cols)
+            assert rows == (128 if m <= 128 else 256) and splits in ((1, 2, 4, 8) if m <= 128 else (1,)), (m, n, rows, splits)
