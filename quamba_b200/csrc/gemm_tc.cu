@@ -356,6 +356,7 @@ gemm_s8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     if (ts.tma_out && lane == 0) bulk_wait_all<0>();
   }
   if (!kPair && ts.splits > 1) {
+    __syncwarp();                             // the producing and the issuing lane come back to their warps: the barrier is .aligned
     cluster_sync();                           // all partial tiles are in shared memory
     int m0, n0;
     tile_at(0, m0, n0);
