@@ -92,7 +92,9 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&r)[32], int m, int 
 // through a swizzled shared-memory buffer and one TMA store, so that global memory sees whole 64- or 128-byte row pieces; rows
 // and columns outside the matrix are dropped by the store.  The fp32 steps and their order are those of Epilogue::scaled.
 // int8: clamp, then round half to even by adding 1.5 * 2^23, whose low mantissa byte is the two's complement result (the
-// conversion pipe, 16 results a clock, is left to the int32 -> fp32 conversions).
+// conversion pipe, 16 results a clock, is left to the int32 -> fp32 conversions).  The clamp would make -128 of a NaN where every
+// other form of the product stores 0, so a piece with a scale that could give one (|acc| <= 2^31: a column scale from 2^96 on can
+// overflow, which times a row scale of 0 is NaN) tests its values; knowing costs one vote per piece of 64 columns.
 constexpr int kOutBuf = 32 * 128;        // bytes of a warp's buffer: 32 rows of 64 fp16 or int8
 __device__ __forceinline__ uint32_t round_s8_bits(float v) { return __float_as_uint(fminf(fmaxf(v, -128.0f), 127.0f) + 12582912.0f); }
 
@@ -100,6 +102,7 @@ __device__ __forceinline__ void store_piece64(const uint32_t (&r0)[32], const ui
                                               uint8_t* buf, int lane, const CUtensorMap* map, int n0, int m0) {
   if (lane == 0) bulk_wait_read<0>();    // the piece before has left the buffer
   __syncwarp();
+  const bool tame = __all_sync(0xffffffffu, fabsf(scale[lane]) < 0x1p96f && fabsf(scale[lane + 32]) < 0x1p96f && fabsf(row_scale) < INFINITY);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -121,6 +124,10 @@ __device__ __forceinline__ void store_piece64(const uint32_t (&r0)[32], const ui
         *reinterpret_cast<uint4*>(buf + lane * 128 + ((p ^ (lane & 7)) << 4)) = w[0];
         *reinterpret_cast<uint4*>(buf + lane * 128 + (((p + 1) ^ (lane & 7)) << 4)) = w[1];
       } else {                           // 64-byte rows: piece p of row r sits at p ^ ((r >> 1) & 3)
+        if (!tame) {
+#pragma unroll
+          for (int t = 0; t < 16; ++t) v[t] = v[t] == v[t] ? v[t] : 0.0f;
+        }
         uint32_t w[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {

@@ -98,3 +98,23 @@ def test_row_and_column_tails_of_every_output(m, per_channel):
             got = ops.w4a8_linear(a, prep, sa.reshape(-1), transpose, out_int8)
             assert torch.equal(got.t() if transpose else got, _convert(want, dtype)), (transpose, dtype)
     ops._lib.read_device_status(torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 512, 256), (65, 9600, 256), (16, 768, 1536), (5, 256, 256)])   # pair, one CTA, K split, dp4a
+def test_scales_that_are_not_finite(m, n, k):
+    """A product that is not a number becomes the int8 0 and an infinite one the end of the range, whichever form the size selects."""
+    a, w, acc, g = _operands(m, k, n)
+    sa, sb = torch.rand((m, 1), device="cuda", generator=g) * 4e-3 + 1e-3, torch.rand((1, n), device="cuda", generator=g) * 4e-3 + 1e-3
+    inf, nan = float("inf"), float("nan")
+    for i, v in enumerate((nan, inf, -inf, 1e38, -3e38)):
+        sb[0, 3 + 17 * i] = v
+        sa[min(i, m - 2), 0] = (nan, inf, -inf, 0.0, 1e38)[i]
+    r = sa * (sb * acc)
+    assert r.isnan().any() and r.isinf().any()
+    want = torch.clamp(torch.round(r), -128, 127).nan_to_num(nan=0.0).to(torch.int8)
+    c = torch.empty((m, n), dtype=torch.int8, device="cuda")
+    ops.quant_linear_cuda.cutlass_scaled_mm_dq(c, a, w.t(), sa, sb)
+    assert torch.equal(c, want)
+    c16 = torch.empty((m, n), dtype=torch.float16, device="cuda")
+    ops.quant_linear_cuda.cutlass_scaled_mm_dq(c16, a, w.t(), sa, sb)
+    assert torch.equal(c16.isnan(), r.isnan()) and torch.equal(c16.nan_to_num(), r.half().nan_to_num())
