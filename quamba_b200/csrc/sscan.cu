@@ -477,10 +477,16 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
     fence_barrier_init();
   }
   __syncwarp();
+  // launched as a programmatic dependent (launch_dependent): the scales may have been written by the kernel before as well
+  grid_dependency_wait();
   auto issue_load = [&](int t, int slot) {
     mbar_arrive_expect_tx(&full[slot], kWTileBytes);
     bulk_load(ring + slot * kWTileBytes, a.state + (int64_t)t * kWTileBytes, kWTileBytes, &full[slot]);
   };
+  if (lane == 0) {
+    issue_load(t_begin, 0);
+    if (t_begin + 1 < t_end) issue_load(t_begin + 1, 1);
+  }
   const int hpg = a.nheads / a.ngroups;
   const float ss0 = kGrouped ? 1.0f : a.state_scale[0];
   const float dt_scale = *a.dt_scale, A_scale = *a.A_scale;
@@ -509,7 +515,8 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
     pos.b = head_lin / a.nheads;
     pos.hd = head_lin % a.nheads;
   }
-  // the row's cell of the grouped scale tables, or 0: constants, looked up one tile ahead as well
+  Raw nxt = fetch(pos);
+  // the row's cell of the grouped scale tables, or 0, looked up one tile ahead as well
   auto cell_of = [&](const Pos& p) {
     if (!kGrouped) return 0;
     const int g = p.hd / hpg, hg = group_lookup(a.head_group_range + g * a.nhead_groups, a.nhead_groups, p.hd % hpg);
@@ -518,13 +525,6 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
   };
   int cell_nxt = cell_of(pos);
   float xs_nxt = a.x_scales[cell_nxt];
-  // launched as a programmatic dependent (launch_dependent): everything above is constant
-  grid_dependency_wait();
-  if (lane == 0) {
-    issue_load(t_begin, 0);
-    if (t_begin + 1 < t_end) issue_load(t_begin + 1, 1);
-  }
-  Raw nxt = fetch(pos);
   f2 bb[8], cc[8];                                            // this lane's slices of B and C, pairs of states
   f2 bs[kGrouped ? 8 : 1], cs[kGrouped ? 8 : 1];              // the same in units of the state scale of `cur_cell`
   int cur_bg = -1, cur_cell = -1, cur_head = -1, slot = 0;

@@ -109,6 +109,7 @@ sscan_cl_kernel(qb_sscan_fwd_args a, int seg_len, int early) {
   extern __shared__ __align__(16) float dyn[];              // per warp 2 x kG x 32 floats of B | C; then the segments' summaries
   __shared__ float s_silu[256];
   if (early) grid_dependency_launch();
+  grid_dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int b = blockIdx.y;                                  // uniform, so that the loads below are uniform base + 32-bit offset
   const int grp = kSeg ? (int)blockIdx.x : (int)blockIdx.x * warps + warp;
@@ -132,7 +133,6 @@ sscan_cl_kernel(qb_sscan_fwd_args a, int seg_len, int early) {
   }
   for (int i = threadIdx.x; i < 256; i += blockDim.x) s_silu[i] = has_z ? silu_mufu(*a.z_scale * (float)(i - 128)) : 1.0f;
   __syncthreads();
-  grid_dependency_wait();
 
   const int8_t* up = a.u + (int64_t)b * a.u_sb;
   const int8_t* dp = a.delta + (int64_t)b * a.delta_sb;
@@ -280,12 +280,12 @@ sscan_cl_wide_kernel(qb_sscan_fwd_args a, int groups, int len_pad, int per, floa
   __shared__ __align__(16) float stage[2 * kWideG * 32];
   __shared__ float s_silu[256];
   if (early) grid_dependency_launch();
+  grid_dependency_wait();
   const int lane = threadIdx.x;
   const int has_z = a.z != nullptr;
   const float su = *a.u_scale, sdt = *a.delta_scale, sA = *a.A_scale;
   for (int i = lane; i < 256; i += 32) s_silu[i] = has_z ? silu_mufu(*a.z_scale * (float)(i - 128)) : 1.0f;
   __syncwarp();
-  grid_dependency_wait();
   // B and C: lane (four rows of eight) reads word lane % 8 of token lane / 8: words 0..3 are B, 4..7 are C
   const bool isC = lane & 4;
   const float bc_scale = isC ? *a.C_scale : *a.B_scale;
