@@ -446,21 +446,27 @@ constexpr int kUpdTileBytes = 8192;
 constexpr int kUpdSlots = 4;
 constexpr int kStatusUpdateLoad = 301;
 
-// Warp-autonomous variant for the Mamba2 decode shape (d_state 128; dt, A, D and the bias tied across a head): every warp owns
-// a ring of kWSlots tiles of 32 state rows (4 KB) and walks a contiguous list of them -- bulk load two tiles ahead, update in
-// place, bulk store -- so no CTA-wide barrier exists after the set-up.  Lane l covers the 16 states n0 = 16 (l & 7) of the rows
-// (l >> 3) + 4 e, e = 0..7.  The states are walked in pairs (packed fp32): 4.5 instructions per state.  What a tile costs
-// besides, a row's x and the sum of its y, is spread over the lanes (lane l owns row (l >> 3) + 4 (l & 7); the eight partial sums
-// of eight rows meet in seven shuffles), and the softplus, the decay and the coordinates are per head.
-// Bound: HBM, two bytes per state.  64 x 80 heads x 64 x 128: 29.5 us with 16-row tiles, scalar arithmetic and per-row
-// scalars (12 instructions per state, issue-bound).
+// Warp-autonomous variant for the Mamba2 decode shape (d_state 128, A tied across the state): every warp owns a ring of kWSlots
+// tiles of kRows state rows and walks a contiguous list of them -- bulk load two tiles ahead, update in place, bulk store -- so no
+// CTA-wide barrier exists after the set-up.  Lane l covers the 16 states n0 = 16 (l & 7) of the rows (l >> 3) + 4 e of a tile.  The
+// states are walked in pairs (packed fp32): 4.5 instructions per state.  What a tile costs besides, a row's x and the sum of its y,
+// is spread over the lanes (lane l owns row (l >> 3) + 4 (l & 7), if the tile has it; the partial sums of a lane's rows meet in seven
+// shuffles), and the coordinates are per head.
+// kTied: dt, A and the bias are one value per head, as the module passes them: softplus and decay are computed once per head.  Else
+// a lane computes them for the row it owns, and the decay goes round with the input (one more shuffle per four rows).  D may be per
+// row in both.
+// kRows: 32, or 16 where the head's rows are a multiple of 16 only.
 // kGrouped: the state scales are a vector per (head group, dim group); a lane keeps B / scale and C * scale of its 16 states for
 // the dim group its rows are in (four consecutive rows of a pass, so they rarely change).
-constexpr int kWTileRows = 32, kWTileBytes = kWTileRows * 128, kWSlots = 3;
-template <bool kGrouped>
+// Bound: HBM, two bytes per state.  64 x 80 heads x 64 x 128, inputs not in L2: 20.5 us (4.1 TB/s) with the scalars of a head, 19.9
+// with D per channel, 21.0 with every scalar per row, where the CTA-tile kernel below takes 36; heads of 48 rows 20.0 against 27.5.
+// (16-row tiles with scalar arithmetic and per-row scalars, the first form, issued 12 instructions per state: 29.5 us.)
+constexpr int kWRows = 32, kWSlots = 3;
+template <bool kGrouped, bool kTied, int kRows>
 __global__ void __launch_bounds__(256, 2)
 sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
   using namespace tc;
+  constexpr int kWTileRows = kRows, kWTileBytes = kRows * 128, kPasses = kRows / 4;
   constexpr float kLog2e = 1.4426950408889634f;
   extern __shared__ __align__(128) uint8_t ring_all[];
   __shared__ __align__(8) uint64_t full_all[8][kWSlots];
@@ -493,7 +499,7 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
   const float bias_scale = (a.dt_bias != nullptr && !a.dt_bias_is_half) ? *a.dt_bias_scale : 0.0f;
   const float D_scale = a.D != nullptr ? *a.D_scale : 0.0f;
   const float z_scale = a.z != nullptr ? *a.z_scale : 0.0f;
-  const int n0 = (lane & 7) * 16, my_row = (lane >> 3) + 4 * (lane & 7);
+  const int n0 = (lane & 7) * 16, my_row = (lane >> 3) + 4 * (lane & (kPasses - 1));   // (16 rows: two lanes hold the same one)
   const int tiles_per_head = a.headdim / kWTileRows;
 
   struct Pos { int b, hd, part; };                            // batch, head, tile within the head
@@ -501,11 +507,21 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
     if (++p.part == tiles_per_head) { p.part = 0; if (++p.hd == a.nheads) { p.hd = 0; ++p.b; } }
     return p;
   };
-  struct Raw { int x, dt; };                                  // inputs written by the kernel before this one, one tile ahead
-  auto fetch = [&](const Pos& p) {
+  struct Raw { int x, dt, A, D; float bias; };                // of the row this lane owns, one tile ahead
+  const bool row_D = a.D != nullptr && (!kTied || a.D_sp != 0);
+  auto bias_at = [&](int hd, int p) {
+    if (a.dt_bias == nullptr) return 0.0f;
+    const int64_t bi = (int64_t)hd * a.bias_sh + (int64_t)p * a.bias_sp;
+    return a.dt_bias_is_half ? __half2float(static_cast<const __half*>(a.dt_bias)[bi]) : bias_scale * (float)static_cast<const int8_t*>(a.dt_bias)[bi];
+  };
+  auto fetch = [&](const Pos& pos) {
     Raw r;
-    r.x = ld_act(a.x + (int64_t)p.b * a.x_sb + (int64_t)p.hd * a.x_sh + p.part * kWTileRows + my_row);
-    r.dt = ld_act(a.dt + (int64_t)p.b * a.dt_sb + (int64_t)p.hd * a.dt_sh);
+    const int p = pos.part * kWTileRows + my_row;
+    r.x = ld_act(a.x + (int64_t)pos.b * a.x_sb + (int64_t)pos.hd * a.x_sh + p);
+    r.dt = ld_act(a.dt + (int64_t)pos.b * a.dt_sb + (int64_t)pos.hd * a.dt_sh + (kTied ? 0 : (int64_t)p * a.dt_sp));
+    r.A = kTied ? 0 : (int)a.A_log[(int64_t)pos.hd * a.A_sh + (int64_t)p * a.A_sp];
+    r.bias = kTied ? 0.0f : bias_at(pos.hd, p);
+    r.D = row_D ? (int)a.D[(int64_t)pos.hd * a.D_sh + (int64_t)p * a.D_sp] : 0;
     return r;
   };
   Pos pos;
@@ -565,26 +581,27 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
       }
       cur_cell = -1;
     }
-    if (cur.b * a.nheads + cur.hd != cur_head) {              // per-head scalars
+    if (!kTied || cur.b * a.nheads + cur.hd != cur_head) {    // once per head, or for the row this lane owns
       cur_head = cur.b * a.nheads + cur.hd;
-      float bias = 0.0f;
-      if (a.dt_bias != nullptr) {
-        const int64_t bi = (int64_t)cur.hd * a.bias_sh;
-        bias = a.dt_bias_is_half ? __half2float(static_cast<const __half*>(a.dt_bias)[bi]) : bias_scale * (float)static_cast<const int8_t*>(a.dt_bias)[bi];
-      }
-      dt = fmaf(dt_scale, (float)raw.dt, bias);
+      dt = fmaf(dt_scale, (float)raw.dt, kTied ? bias_at(cur.hd, 0) : raw.bias);
       if (a.dt_softplus) dt = softplus_f(dt);
-      dA = fast_exp2(-__expf(A_scale * (float)a.A_log[(int64_t)cur.hd * a.A_sh]) * kLog2e * dt);
-      dskip = a.D != nullptr ? D_scale * (float)a.D[(int64_t)cur.hd * a.D_sh] : 0.0f;
+      const int Aq = kTied ? (int)a.A_log[(int64_t)cur.hd * a.A_sh] : raw.A;
+      dA = fast_exp2(-__expf(A_scale * (float)Aq) * kLog2e * dt);
+      if (!row_D) dskip = a.D != nullptr ? D_scale * (float)a.D[(int64_t)cur.hd * a.D_sh] : 0.0f;
     }
+    if (row_D) dskip = D_scale * (float)raw.D;
     const float x = xs * (float)raw.x, dtx = dt * x;          // of row my_row
-    const f2 dA2 = pack2(dA, dA);
+    f2 dA2 = pack2(dA, dA);
     if (!mbar_wait(&full[slot], phase, status, kStatusUpdateLoad)) break;   // all lanes wait on it
     uint8_t* tile = ring + slot * kWTileBytes;
-    float y[8];
+    float y[kPasses];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < kPasses; ++e) {
       const int r = (lane >> 3) + 4 * e;                      // owned by lane e of this lane's eight
+      if (!kTied) {
+        const float dA_r = __shfl_sync(0xffffffffu, dA, e, 8);
+        dA2 = pack2(dA_r, dA_r);
+      }
       const float dtx_r = __shfl_sync(0xffffffffu, dtx, e, 8);
       const f2 dtx2 = pack2(dtx_r, dtx_r);
       if (kGrouped) {
@@ -635,10 +652,14 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
       bulk_wait_read<1>();      // every store but the newest has finished reading its slot
       if (t + 2 < t_end) issue_load(t + 2, slot == 0 ? 2 : slot - 1);
     }
-    // eight rows' partial sums over eight lanes: halve the rows a lane carries while adding its partner's, until lane e of the
-    // eight holds the row it owns
+    // the partial sums of kPasses rows over eight lanes: halve the rows a lane carries while adding its partner's, until each lane
+    // holds the row it owns
+    if (kPasses == 4) {
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
+      for (int i = 0; i < kPasses; ++i) y[i] += __shfl_xor_sync(0xffffffffu, y[i], 4);
+    }
+#pragma unroll
+    for (int o = kPasses / 2; o > 0; o >>= 1) {
       const bool hi = lane & o;
 #pragma unroll
       for (int i = 0; i < o; ++i) {
@@ -652,10 +673,23 @@ sscan_update_warp_kernel(qb_sscan_update_args a, int tiles, int* status) {
       const float z = z_scale * (float)ld_act(a.z + (int64_t)cur.b * a.z_sb + (int64_t)cur.hd * a.z_sh + p);
       yv *= silu_exact(z);
     }
-    static_cast<__half*>(a.out)[(int64_t)cur.b * a.out_sb + (int64_t)cur.hd * a.out_sh + p] = __float2half_rn(yv);
+    if (kPasses == 8 || (lane & 4) == 0)
+      static_cast<__half*>(a.out)[(int64_t)cur.b * a.out_sb + (int64_t)cur.hd * a.out_sh + p] = __float2half_rn(yv);
     if (++slot == kWSlots) { slot = 0; phase ^= 1; }
   }
   if (lane == 0) bulk_wait_all<0>();
+}
+
+template <bool kGrouped, bool kTied, int kRows>
+int launch_update_warp(const qb_sscan_update_args& a, int* status, cudaStream_t st) {
+  constexpr int smem = 8 * kWSlots * kRows * 128;
+  static PerDeviceOnce attr;
+  if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_warp_kernel<kGrouped, kTied, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int tiles = (int)((int64_t)a.batch * a.nheads * a.headdim / kRows);
+  const dim3 grid((unsigned)std::min<int64_t>(ceil_div(tiles, 8), (int64_t)sm_count() * 2));
+  launch_dependent(sscan_update_warp_kernel<kGrouped, kTied, kRows>, grid, dim3(256), smem, st, a, tiles, status);
+  QB_LAUNCH_OK("sscan_update_warp_kernel");
+  return QB_OK;
 }
 
 template <int LPR, bool kTied, bool kGrouped>
@@ -943,7 +977,6 @@ extern "C" int qb_sscan_update(const qb_sscan_update_args* a, void* stream) {
   QB_REQUIRE(a->nheads % a->ngroups == 0, QB_ERR_INVALID_ARG, "nheads must be divisible by ngroups");
   QB_REQUIRE(!a->grouped || (a->head_group_range && a->dim_group_range && a->nhead_groups > 0 && a->ndim_groups > 0),
              QB_ERR_INVALID_ARG, "sscan_update: grouped scales need the range tables");
-  // warp-autonomous kernel: the Mamba2 decode shape (d_state 128, A tied across the state, per-tensor scales), fully
   // few (batch, head) pairs: the low-latency kernel, one CTA per pair
   if (a->dstate == 128 && a->A_sn == 0 && a->A_sp == 0 && a->dt_sp == 0 && !a->grouped && a->z == nullptr && a->headdim % 64 == 0 &&
       (a->D == nullptr || a->D_sp == 0) && (a->dt_bias == nullptr || a->bias_sp == 0) && a->state_sp % 16 == 0 && a->state_sh % 16 == 0 &&
@@ -956,29 +989,22 @@ extern "C" int qb_sscan_update(const qb_sscan_update_args* a, void* stream) {
   }
   QB_REQUIRE(!a->early_launch, QB_ERR_UNSUPPORTED,
              "sscan_update: early_launch is only offered on the one-CTA-per-head decode kernel, which this call is not eligible for");
-  // contiguous state, 32-row tiles inside one head, scalars tied across it (grouped scales: from 512 tiles on; below that the
-  // CTA-tile kernel's shorter set-up wins, 6.7 against 7.9 us for 2 x 24 heads)
-  if (a->dstate == 128 && a->A_sn == 0 && a->A_sp == 0 && a->dt_sp == 0 && (a->D == nullptr || a->D_sp == 0) &&
-      (a->dt_bias == nullptr || a->bias_sp == 0) && (!a->grouped || (aligned(a->state_scale, 16) && (int64_t)a->batch * a->nheads * a->headdim >= 512 * kWTileRows)) && a->headdim % kWTileRows == 0 && aligned(a->state, 16) &&
-      a->state_sp == a->dstate && a->state_sh == (int64_t)a->headdim * a->dstate &&
-      a->state_sb == (int64_t)a->nheads * a->headdim * a->dstate && aligned(a->Bm, 16) && aligned(a->Cm, 16) &&
-      a->B_sb % 16 == 0 && a->B_sg % 16 == 0 && a->C_sb % 16 == 0 && a->C_sg % 16 == 0 &&
+  // contiguous state of d_state 128, A tied across it, tiles of 32 or 16 rows inside one head
+  const bool tied = a->A_sp == 0 && a->dt_sp == 0 && (a->dt_bias == nullptr || a->bias_sp == 0) && a->headdim % kWRows == 0;
+  // grouped scales: with the scalars of a head, from 512 tiles on; below that the CTA-tile kernel's shorter set-up wins, 6.7
+  // against 7.9 us for 2 x 24 heads
+  const bool warp_tiles = a->grouped ? tied && aligned(a->state_scale, 16) && (int64_t)a->batch * a->nheads * a->headdim >= 512 * kWRows
+                                     : a->headdim % 16 == 0;
+  if (warp_tiles && a->dstate == 128 && a->A_sn == 0 && aligned(a->state, 16) && a->state_sp == a->dstate &&
+      a->state_sh == (int64_t)a->headdim * a->dstate && a->state_sb == (int64_t)a->nheads * a->headdim * a->dstate &&
+      aligned(a->Bm, 16) && aligned(a->Cm, 16) && a->B_sb % 16 == 0 && a->B_sg % 16 == 0 && a->C_sb % 16 == 0 && a->C_sg % 16 == 0 &&
       !path_override(QB_PATH_UPDATE_CTA_TILES)) {
     int* status = device_status_ptr();
     QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "sscan_update: device status word unavailable");
-    static PerDeviceOnce wattr;
-    constexpr int wsmem = 8 * kWSlots * kWTileBytes;
-    if (wattr.first()) {
-      QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_warp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
-      QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_warp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
-    }
-    const int64_t rows = (int64_t)a->batch * a->nheads * a->headdim;
-    const int wtiles = (int)(rows / kWTileRows);
-    const dim3 grid((unsigned)std::min<int64_t>(ceil_div(wtiles, 8), (int64_t)sm_count() * 2));
-    if (a->grouped) launch_dependent(sscan_update_warp_kernel<true>, grid, dim3(256), wsmem, (cudaStream_t)stream, *a, wtiles, status);
-    else launch_dependent(sscan_update_warp_kernel<false>, grid, dim3(256), wsmem, (cudaStream_t)stream, *a, wtiles, status);
-    QB_LAUNCH_OK("sscan_update_warp_kernel");
-    return QB_OK;
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (a->grouped) return launch_update_warp<true, true, kWRows>(*a, status, st);
+    if (tied) return launch_update_warp<false, true, kWRows>(*a, status, st);
+    return a->headdim % kWRows == 0 ? launch_update_warp<false, false, kWRows>(*a, status, st) : launch_update_warp<false, false, 16>(*a, status, st);
   }
   // pipelined kernel: fully contiguous state, dstate in {16, 32, 64, 128, 256}, whole 8 KB tiles inside one (batch, group)
   {

@@ -386,8 +386,8 @@ def test_no_device_wait_timed_out():
 
 # ---- state update: the kernels behind qb_sscan_update (warp-autonomous, pipelined bulk-copy, streaming, generic) -----
 @pytest.mark.parametrize("Bsz,H,P,G,N,grouped,layout", [
-    (3, 8, 64, 1, 128, False, "contig"),     # Mamba2 decode shape: warp-autonomous kernel (16-row tiles)
-    (7, 5, 48, 1, 128, False, "contig"),     # the same kernel: three tiles per head, 105 tiles over the warps
+    (3, 8, 64, 1, 128, False, "contig"),     # d_state 128, scalars per row: warp-autonomous kernel, 32-row tiles
+    (7, 5, 48, 1, 128, False, "contig"),     # the same kernel: three 16-row tiles per head, 105 tiles over the warps
     (4, 6, 32, 2, 128, False, "contig"),     # the same kernel: two SSD groups
     (2, 8, 64, 2, 128, True, "contig"),      # pipelined, grouped scales
     (2, 4, 64, 1, 256, False, "contig"),     # pipelined, 16 pieces per row
@@ -437,8 +437,7 @@ def test_update_kernel_variants_against_oracle(Bsz, H, P, G, N, grouped, layout)
     ops()._lib.read_device_status(torch.cuda.current_stream().cuda_stream)      # raises if a device-side wait timed out
 
 
-# ---- large GEMMs: the persistent tensor-core kernel (needs at least one 128 x 256 tile per SM; the tile width it then
-# uses, 192 or 256 columns, depends on the shape: the cases below reach both) ---------------------------
+# ---- large GEMMs: CTA pairs on 256-row tiles, whose width depends on the shape ------------------------
 @pytest.mark.parametrize("M,K,N,out_dtype", [(2000, 528, 3024, torch.int8), (2048, 1024, 5120, torch.float16),
                                              (4100, 272, 2304, torch.int8), (2048, 512, 2560, torch.float16),
                                              (2048, 256, 10576, torch.int8), (8192, 128, 2560, torch.float16)])

@@ -87,6 +87,20 @@ def test_scalars_of_a_head(B, H, P, G, z, D, grouped):
     _check(_case(B, H, P, G, grouped, z=z, D=D), "sscan_update_warp_kernel")
 
 
+@pytest.mark.parametrize("B,H,P,G,z,dt,bias,i8_bias,A,D", [
+    (8, 80, 64, 1, False, "head", "head", False, "head", "row"),          # D per channel, the rest per head
+    (8, 80, 64, 2, True, "row", "head", True, "head", "head"), (7, 45, 96, 1, False, "head", "row", True, "head", "row"),
+    (6, 51, 32, 1, False, "head", "head", False, "row", None), (9, 24, 64, 8, True, "row", "row", False, "row", "row"),
+    (7, 43, 48, 1, False, "head", "head", False, "head", "head"), (5, 30, 16, 2, True, "row", "row", True, "row", "row"),    # 16-row tiles
+    (1, 1, 48, 1, False, "row", "row", False, "row", "row")])
+def test_scalars_of_a_row(B, H, P, G, z, dt, bias, i8_bias, A, D):
+    _check(_case(B, H, P, G, False, seed=1, z=z, D=D, dt=dt, bias=bias, i8_bias=i8_bias, A=A), "sscan_update_warp_kernel")
+
+
+def test_channel_D_with_grouped_scales():
+    _check(_case(8, 80, 64, 1, True, seed=2, D="row"), "sscan_update_warp_kernel")
+
+
 @pytest.mark.parametrize("grouped", [False, True])
 def test_scales_written_by_the_launch_before(grouped):
     """The update is launched as a programmatic dependent; scales that the kernel before it on the stream writes last are its scales."""
