@@ -237,7 +237,9 @@ PyObject* sscan_update(const Args& a) {
   need(st.dim() == 4 && x.dim() == 3 && B.dim() == 3, "state must be (batch, [nheads,] dim, dstate)");
   const int64_t groups = B.size(1), batch = st.size(0), nh = st.size(1), dim = st.size(2), n = st.size(3);
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
-  need(x.is_cuda(), "q_x must be a CUDA tensor");
+  cuda_i8(st, "state"); cuda_i8(x, "q_x");
+  cuda_f32(xs, "x_scales"); cuda_f32(ss, "ssm_state_scale"); cuda_f32(a.tensor(6), "dt_scale"); cuda_f32(a.tensor(8), "A_log_scale");
+  cuda_f32(a.tensor(11), "B_scale"); cuda_f32(a.tensor(13), "C_scale");
   need(is(x, {batch, nh, dim}), "q_x must have shape (batch, nheads, dim)");
   need(dt.sizes() == x.sizes(), "q_dt must have the shape of q_x");
   need(is(A, {nh, dim, n}), "q_A_log must have shape (nheads, dim, dstate)");
@@ -301,6 +303,8 @@ PyObject* ssd(const Args& a) {
   const int64_t batch = x.size(0), len = x.size(1), nh = x.size(2), hd = x.size(3), groups = B.size(2), n = B.size(3);
   need(groups > 0 && nh % groups == 0, "nheads must be divisible by ngroups");
   cuda_i8(x, "q_x"); cuda_i8(B, "q_B"); cuda_i8(dt, "q_dt"); cuda_i8(A, "q_A_log"); cuda_i8(C, "q_C");
+  cuda_f32(xs, "x_scales"); cuda_f32(ss, "ssm_state_scale"); cuda_f32(a.tensor(5), "dt_scale"); cuda_f32(a.tensor(7), "A_log_scale");
+  cuda_f32(Bs, "B_scale"); cuda_f32(Cs, "C_scale");
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
   need(is(B, {batch, len, groups, n}) && C.sizes() == B.sizes(), "q_B / q_C shape mismatch");
   need(is(dt, {batch, len, nh}), "q_dt must be (batch, seqlen, nheads)");
@@ -435,6 +439,7 @@ void check_norm(const Tensor& x, const Tensor& w, const Tensor& bias) {
   need(x.is_cuda() && x.scalar_type() == at::kHalf && x.dim() == 2, "x must be a 2-D float16 CUDA tensor");
   need(x.stride(-1) == 1, "x must be contiguous in its last dim");
   const int64_t n = x.size(1);
+  need(w.is_cuda(), "weight must be a CUDA tensor");
   need(w.dim() == 1 && w.size(0) == n && w.stride(0) == 1 && w.scalar_type() == at::kHalf, "weight must be fp16 (N,)");
   if (bias.defined()) need(bias.dim() == 1 && bias.size(0) == n && bias.stride(0) == 1 && bias.scalar_type() == at::kHalf, "bias must be fp16 (N,)");
 }

@@ -31,6 +31,9 @@ inline void cuda_i8(const Tensor& t, const char* name) {
   if (!t.is_cuda()) throw std::runtime_error(std::string(name) + " must be a CUDA tensor");
   if (t.scalar_type() != at::kChar) throw std::runtime_error(std::string(name) + " must be int8");
 }
+inline void cuda_f32(const Tensor& t, const char* name) {
+  if (!t.is_cuda() || t.scalar_type() != at::kFloat) throw std::runtime_error(std::string(name) + " must be a float32 CUDA tensor");
+}
 inline Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline int8_t* i8(const Tensor& t) { return static_cast<int8_t*>(ptr(t)); }
@@ -120,6 +123,11 @@ PyObject* entry(PyObject*, PyObject* const* v, Py_ssize_t n) {
 // Attribute names are interned once; a lookup is then a pointer-keyed dictionary probe.
 #define QBN_NAME(x) ([]() -> PyObject* { static PyObject* s = PyUnicode_InternFromString(#x); return s; }())
 
+inline const Tensor& plain(const Tensor& t, at::ScalarType type, c10::Device dev) {
+  if (t.scalar_type() != type || t.device() != dev) throw NotPlain{};
+  return t;
+}
+
 // A torch.nn.Module as its dictionaries: plain attributes, buffers, sub-modules.
 struct Mod {
   PyObject* self;
@@ -139,6 +147,12 @@ struct Mod {
   Tensor opt_tensor(PyObject* name) const {
     PyObject* r = get(name);
     return r == Py_None ? Tensor() : as_tensor(r);
+  }
+  // of the given type on the given device, as the kernels read it; anything else is for the module walk (and its errors)
+  Tensor tensor_on(PyObject* name, at::ScalarType type, c10::Device dev) const { return plain(tensor(name), type, dev); }
+  Tensor opt_tensor_on(PyObject* name, at::ScalarType type, c10::Device dev) const {
+    const Tensor t = opt_tensor(name);
+    return t.defined() ? plain(t, type, dev) : t;
   }
   double num(PyObject* name) const { return as_double(get(name)); }
   double num_or(PyObject* name, double d) const {

@@ -60,6 +60,7 @@ Mod Mod::child(PyObject* name, PyTypeObject* type) const {
 }
 
 void Conv2::check() {
+  cuda_f32(out_scale[0], "x_scales"); cuda_f32(out_scale[1], "B_scales"); cuda_f32(out_scale[2], "C_scales");
   if (hgr.defined() && dgr.defined()) {
     need(hgr.scalar_type() == at::kInt && dgr.scalar_type() == at::kInt, "group ranges must be int32");
     need(hgr.size(0) == groups && dgr.size(0) == groups, "x_head_group_range.shape[0] / x_dim_group_range.shape[0] must equal the number of groups");
@@ -136,7 +137,7 @@ struct Lin {
   Mod m;
   int64_t k, n, features;
   bool w4, int8;
-  Lin(const Mod& parent, PyObject* name) : m(open(parent, name)) {
+  Lin(const Mod& parent, PyObject* name, c10::Device dev) : m(open(parent, name)) {
     const Types& t = g_types;
     PyTypeObject* ty = Py_TYPE(m.self);
     w4 = ty == t.W4A8B16O16Linear || ty == t.W4A8B8O8Linear || ty == t.W4A8B8O8LinearParallel;
@@ -147,10 +148,12 @@ struct Lin {
     n = features + m.integer(QBN_NAME(pad_out));
     if (w4) {
       if (m.integer(QBN_NAME(size_n)) != n || m.integer(QBN_NAME(size_k)) != k) throw NotPlain{};
+      m.tensor_on(QBN_NAME(weight), at::kInt, dev);
+      m.tensor_on(QBN_NAME(input_scale), at::kFloat, dev);
     } else {
-      const Tensor w = m.tensor(QBN_NAME(weight)), sa = m.tensor(QBN_NAME(a)), sb = m.tensor(QBN_NAME(b));
+      const Tensor w = m.tensor_on(QBN_NAME(weight), at::kChar, dev), sa = m.tensor_on(QBN_NAME(a), at::kFloat, dev), sb = m.tensor_on(QBN_NAME(b), at::kFloat, dev);
       if (w.dim() != 2 || w.size(0) != k || w.size(1) != n || w.stride(0) != 1 || w.stride(1) % 16 != 0 || !sa.is_contiguous() || !sb.is_contiguous() ||
-          sa.scalar_type() != at::kFloat || sb.scalar_type() != at::kFloat || sa.numel() != 1 || (sb.numel() != 1 && sb.numel() != n))
+          sa.numel() != 1 || (sb.numel() != 1 && sb.numel() != n))
         throw NotPlain{};
     }
   }
@@ -208,15 +211,15 @@ struct BlockNorm {
   BlockNorm(PyObject* norm, const Tensor& x, PyObject* res_obj, bool fp32, int64_t m, int64_t n, const Device& dev) {
     Mod nm(norm);
     nm.require_plain(g_types.QRMSNorm);
-    const Tensor w = nm.tensor(QBN_NAME(weight)), bias = nm.opt_tensor(QBN_NAME(bias));
+    const Tensor w = nm.tensor_on(QBN_NAME(weight), at::kHalf, dev.dev), bias = nm.opt_tensor(QBN_NAME(bias));
     const double scale = nm.num_or(QBN_NAME(output_scale), 0.0);
-    if (scale == 0.0 || bias.defined() || w.numel() != n || w.scalar_type() != at::kHalf || !w.is_contiguous() || x.scalar_type() != at::kHalf || n * 2 >= 65536)
+    if (scale == 0.0 || bias.defined() || w.numel() != n || !w.is_contiguous() || x.scalar_type() != at::kHalf || n * 2 >= 65536)
       throw NotPlain{};
     qb_rmsnorm_args s{};
     bool f32_out = fp32;
     if (res_obj != Py_None) {
       const Tensor r = as_tensor(res_obj);
-      if (r.sizes() != x.sizes() || !r.is_contiguous() || (r.scalar_type() != at::kHalf && r.scalar_type() != at::kFloat)) throw NotPlain{};
+      if (r.sizes() != x.sizes() || r.device() != x.device() || !r.is_contiguous() || (r.scalar_type() != at::kHalf && r.scalar_type() != at::kFloat)) throw NotPlain{};
       f32_out = r.scalar_type() == at::kFloat;
       s.residual = r.data_ptr(); s.residual_row_stride = n; s.residual_is_f32 = f32_out;
     }
@@ -272,7 +275,8 @@ PyObject* mamba2_layer(const Args& a) {
   if (!x.is_cuda() || x.dim() != 3 || !x.is_contiguous() || x.numel() == 0) throw NotPlain{};
   const int64_t batch = x.size(0), len = x.size(1), dm = x.size(2), rows = batch * len;
   if (decode && len != 1) throw NotPlain{};
-  const Lin in(mx, QBN_NAME(in_proj)), outp(mx, QBN_NAME(out_proj));
+  const c10::Device on = x.device();
+  const Lin in(mx, QBN_NAME(in_proj), on), outp(mx, QBN_NAME(out_proj), on);
   const Mod conv = mx.child(QBN_NAME(conv1d), g_types.Quamb2Conv1D), scan = mx.child(QBN_NAME(qchunk_scan), g_types.Quamba2ChunkScan),
             gn_m = mx.child(QBN_NAME(norm), g_types.QRMSNormGated), had_m = mx.child(QBN_NAME(had), g_types.QHadamard);
   const int64_t d = mx.integer(QBN_NAME(d_ssm)), groups = mx.integer(QBN_NAME(ngroups)), ds = mx.integer(QBN_NAME(d_state)),
@@ -282,19 +286,19 @@ PyObject* mamba2_layer(const Args& a) {
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
   if (decode && !conv_st.defined()) throw NotPlain{};
   if (conv_st.defined() && (conv_st.scalar_type() != at::kChar || !is(conv_st, {batch, dim, 4}) || ssm_st.scalar_type() != at::kChar ||
-                            !is(ssm_st, {batch, nh, hd, ds}) || !ssm_st.is_contiguous() || conv_st.device() != x.device() ||
+                            !is(ssm_st, {batch, nh, hd, ds}) || !ssm_st.is_contiguous() || conv_st.device() != on || ssm_st.device() != on ||
                             (conv_st.stride(1) == 1 && (conv_st.stride(0) % 4 != 0 || conv_st.stride(2) % 4 != 0 || reinterpret_cast<uintptr_t>(conv_st.data_ptr()) % 4 != 0))))
     throw NotPlain{};
 
   Conv2 c;
-  c.weight = conv.tensor(QBN_NAME(weight)); c.bias = conv.opt_tensor(QBN_NAME(bias));
-  c.hgr = conv.opt_tensor(QBN_NAME(x_head_group_range)); c.dgr = conv.opt_tensor(QBN_NAME(x_dim_group_range));
+  c.weight = conv.tensor_on(QBN_NAME(weight), at::kChar, on); c.bias = conv.opt_tensor_on(QBN_NAME(bias), at::kChar, on);
+  c.hgr = conv.opt_tensor_on(QBN_NAME(x_head_group_range), at::kInt, on); c.dgr = conv.opt_tensor_on(QBN_NAME(x_dim_group_range), at::kInt, on);
   PyObject* so[3] = {QBN_NAME(x_out_scales), QBN_NAME(B_out_scales), QBN_NAME(C_out_scales)};
   PyObject* si[3] = {QBN_NAME(x_scale), QBN_NAME(B_scale), QBN_NAME(C_scale)};
   PyObject* sw[3] = {QBN_NAME(wx_scale), QBN_NAME(wB_scale), QBN_NAME(wC_scale)};
   PyObject* sb[3] = {QBN_NAME(bx_scale), QBN_NAME(bB_scale), QBN_NAME(bC_scale)};
   for (int i = 0; i < 3; ++i) {
-    c.out_scale[i] = conv.tensor(so[i]);
+    c.out_scale[i] = conv.tensor_on(so[i], at::kFloat, on);
     c.in[i] = conv.num(si[i]); c.w_scale[i] = conv.num(sw[i]); c.b_scale[i] = conv.num_or(sb[i], 0.0);
   }
   c.x_dim = conv.integer(QBN_NAME(x_dim)); c.headdim = conv.integer(QBN_NAME(x_headdim)); c.d_state = conv.integer(QBN_NAME(d_state));
@@ -303,22 +307,22 @@ PyObject* mamba2_layer(const Args& a) {
     throw NotPlain{};
   c.check();
 
-  const Tensor A = scan.tensor(QBN_NAME(A_log)), D = scan.opt_tensor(QBN_NAME(D)), bias = scan.opt_tensor(QBN_NAME(dt_bias)),
-               ss = scan.tensor(QBN_NAME(ssm_state_scale)), xs = scan.tensor(QBN_NAME(x_scales)), Bs = scan.tensor(QBN_NAME(B_scale)),
-               Cs = scan.tensor(QBN_NAME(C_scale)), dts = scan.tensor(QBN_NAME(dt_scale)), As = scan.tensor(QBN_NAME(A_log_scale)),
-               hgr = scan.opt_tensor(QBN_NAME(x_head_group_range)), dgr = scan.opt_tensor(QBN_NAME(x_dim_group_range));
-  const Tensor Ds = D.defined() ? scan.tensor(QBN_NAME(D_scale)) : Tensor();
+  auto scale = [&](PyObject* name) { return scan.tensor_on(name, at::kFloat, on); };
+  const Tensor A = scan.tensor_on(QBN_NAME(A_log), at::kChar, on), D = scan.opt_tensor_on(QBN_NAME(D), at::kChar, on),
+               bias = scan.opt_tensor_on(QBN_NAME(dt_bias), at::kHalf, on), ss = scale(QBN_NAME(ssm_state_scale)), xs = scale(QBN_NAME(x_scales)),
+               Bs = scale(QBN_NAME(B_scale)), Cs = scale(QBN_NAME(C_scale)), dts = scale(QBN_NAME(dt_scale)), As = scale(QBN_NAME(A_log_scale)),
+               hgr = scan.opt_tensor_on(QBN_NAME(x_head_group_range), at::kInt, on), dgr = scan.opt_tensor_on(QBN_NAME(x_dim_group_range), at::kInt, on);
+  const Tensor Ds = D.defined() ? scale(QBN_NAME(D_scale)) : Tensor();
   const bool hdim = scan.flag(QBN_NAME(D_has_hdim)), grouped = hgr.defined();
   if (A.numel() != nh || !A.is_contiguous() || (D.defined() && (D.numel() != (hdim ? d : nh) || !D.is_contiguous())) ||
-      (bias.defined() && (bias.scalar_type() != at::kHalf || bias.numel() != nh || !bias.is_contiguous())) || grouped != dgr.defined() ||
+      (bias.defined() && (bias.numel() != nh || !bias.is_contiguous())) || grouped != dgr.defined() ||
       (grouped && (!hgr.is_contiguous() || !dgr.is_contiguous() || hgr.dim() != 2 || dgr.dim() != 3 || !is(ss, {groups, hgr.size(1), dgr.size(2), ds}) || !ss.is_contiguous() ||
-                   xs.numel() != groups * hgr.size(1) * dgr.size(2) || Bs.numel() != groups || Cs.numel() != groups || hgr.scalar_type() != at::kInt ||
-                   dgr.scalar_type() != at::kInt)) ||
+                   xs.numel() != groups * hgr.size(1) * dgr.size(2) || Bs.numel() != groups || Cs.numel() != groups)) ||
       (!grouped && (xs.numel() != 1 || Bs.numel() != 1 || Cs.numel() != 1 || ss.numel() != 1)))
     throw NotPlain{};
-  const Tensor gw = gn_m.tensor(QBN_NAME(weight));
+  const Tensor gw = gn_m.tensor_on(QBN_NAME(weight), at::kHalf, on);
   const int64_t gsize = gn_m.get(QBN_NAME(group_size)) == Py_None ? d : gn_m.integer(QBN_NAME(group_size));
-  if (!gn_m.flag(QBN_NAME(use_float16_output)) || gn_m.get(QBN_NAME(bias)) != Py_None || gw.numel() != d || gw.scalar_type() != at::kHalf || !gw.is_contiguous() ||
+  if (!gn_m.flag(QBN_NAME(use_float16_output)) || gn_m.get(QBN_NAME(bias)) != Py_None || gw.numel() != d || !gw.is_contiguous() ||
       gsize <= 0 || d % gsize != 0)
     throw NotPlain{};
   PyObject* lim = scan.get(QBN_NAME(dt_limit));
@@ -409,7 +413,8 @@ PyObject* mamba1_layer(const Args& a) {
   if (!x.is_cuda() || x.dim() != 3 || !x.is_contiguous() || x.numel() == 0) throw NotPlain{};
   const int64_t batch = x.size(0), len = x.size(1), dm = x.size(2), rows = batch * len;
   if (decode && len != 1) throw NotPlain{};
-  const Lin in(mx, QBN_NAME(in_proj)), xp(mx, QBN_NAME(x_proj)), dtp(mx, QBN_NAME(dt_proj)), outp(mx, QBN_NAME(out_proj));
+  const c10::Device on = x.device();
+  const Lin in(mx, QBN_NAME(in_proj), on), xp(mx, QBN_NAME(x_proj), on), dtp(mx, QBN_NAME(dt_proj), on), outp(mx, QBN_NAME(out_proj), on);
   const Mod conv = mx.child(QBN_NAME(conv1d), g_types.QCausalConv1D), scan = mx.child(QBN_NAME(selective_scan), g_types.QSScan),
             had_m = mx.child(QBN_NAME(had), g_types.QHadamard);
   const int64_t d = mx.integer(QBN_NAME(d_inner)), ds = mx.integer(QBN_NAME(d_state)), rank = mx.integer(QBN_NAME(dt_rank));
@@ -418,21 +423,25 @@ PyObject* mamba1_layer(const Args& a) {
     throw NotPlain{};
   const Tensor conv_st = a.opt_tensor(5), ssm_st = a.opt_tensor(6);
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
-  const Tensor cw = conv.tensor(QBN_NAME(weight)), cb = conv.opt_tensor(QBN_NAME(bias));
+  const Tensor cw = conv.tensor_on(QBN_NAME(weight), at::kChar, on), cb = conv.opt_tensor_on(QBN_NAME(bias), at::kChar, on);
   if (decode && !conv_st.defined()) throw NotPlain{};
   if (cw.dim() != 2 || cw.size(0) != d || cw.size(1) != 4 || !cw.is_contiguous() || (cb.defined() && !cb.is_contiguous()) ||
       (conv_st.defined() && (conv_st.scalar_type() != at::kChar || !is(conv_st, {batch, d, 4}) || ssm_st.scalar_type() != at::kChar ||
-                             !is(ssm_st, {batch, d, ds}) || !ssm_st.is_contiguous() || conv_st.device() != x.device() ||
+                             !is(ssm_st, {batch, d, ds}) || !ssm_st.is_contiguous() || conv_st.device() != on || ssm_st.device() != on ||
                              (conv_st.stride(1) == 1 && (conv_st.stride(0) % 4 != 0 || conv_st.stride(2) % 4 != 0)))))
     throw NotPlain{};
-  const Tensor A = scan.tensor(QBN_NAME(A_log)), D = scan.opt_tensor(QBN_NAME(D)), bias = scan.opt_tensor(QBN_NAME(dt_bias));
-  const Tensor As = scan.tensor(QBN_NAME(A_scale)), us = scan.tensor(QBN_NAME(u_scale)), dts = scan.tensor(QBN_NAME(dt_scale)), Bs = scan.tensor(QBN_NAME(B_scale)),
-               Cs = scan.tensor(QBN_NAME(C_scale)), zs = scan.tensor(QBN_NAME(z_scale)), ss = scan.tensor(QBN_NAME(ssm_state_scale));
-  const Tensor Ds = scan.tensor(QBN_NAME(D_scale)), bs = scan.tensor(QBN_NAME(dt_bias_scale));
-  for (const Tensor* t : {&As, &us, &dts, &Bs, &Cs, &zs, &ss, &Ds, &bs})
-    if (t->numel() != 1 || t->scalar_type() != at::kFloat || !t->is_cuda()) throw NotPlain{};
-  if (!is(A, {d, ds}) || !A.is_contiguous() || A.scalar_type() != at::kChar || (D.defined() && (D.numel() != d || !D.is_contiguous())) ||
-      (bias.defined() && (bias.numel() != d || !bias.is_contiguous() || bias.scalar_type() != at::kChar)))
+  const Tensor A = scan.tensor_on(QBN_NAME(A_log), at::kChar, on), D = scan.opt_tensor_on(QBN_NAME(D), at::kChar, on),
+               bias = scan.opt_tensor_on(QBN_NAME(dt_bias), at::kChar, on);
+  auto scale = [&](PyObject* name) {
+    const Tensor t = scan.tensor_on(name, at::kFloat, on);
+    if (t.numel() != 1) throw NotPlain{};
+    return t;
+  };
+  const Tensor As = scale(QBN_NAME(A_scale)), us = scale(QBN_NAME(u_scale)), dts = scale(QBN_NAME(dt_scale)), Bs = scale(QBN_NAME(B_scale)),
+               Cs = scale(QBN_NAME(C_scale)), zs = scale(QBN_NAME(z_scale)), ss = scale(QBN_NAME(ssm_state_scale)), Ds = scale(QBN_NAME(D_scale)),
+               bs = scale(QBN_NAME(dt_bias_scale));
+  if (!is(A, {d, ds}) || !A.is_contiguous() || (D.defined() && (D.numel() != d || !D.is_contiguous())) ||
+      (bias.defined() && (bias.numel() != d || !bias.is_contiguous())))
     throw NotPlain{};
   const Rotation had(had_m);
   if (had.blocks <= 0 || d % had.blocks != 0) throw NotPlain{};

@@ -81,3 +81,55 @@ def test_mamba1_channel_last_layer_against_the_module_walk(weights, batch, lengt
     assert (ya - yb).norm() <= 0.02 * yb.norm()
     diff = (sa.int() - sb.int()).abs()
     assert diff.max() <= 1 and (diff != 0).float().mean() <= 2e-3
+
+
+def _mamba1_layer(weights):
+    from quamba_b200 import calibrate as cal
+    fm = cal.Mamba1LMFloat(d_model=256, n_layer=1, vocab_size=320, seed=6, w4_group_size=None if weights == "w8" else 128)
+    ids = torch.randint(0, 320, (1, 48), generator=torch.Generator().manual_seed(6))
+    return cal.quantize_mamba1_model(fm, [ids], w_bits=int(weights[1])).to("cuda").backbone.layers[0]
+
+
+def _any_layer(family, weights):
+    return _layer(weights, False) if family == "mamba2" else _mamba1_layer(weights)
+
+
+def _call(layer, batch, length, decode, caches=None):
+    g = torch.Generator(device="cuda").manual_seed(length)
+    params = InferenceParams(max_seqlen=8, max_batch_size=batch, seqlen_offset=int(decode))
+    params.key_value_memory_dict[0] = caches if caches is not None else layer.allocate_inference_cache(batch, 8)
+    out, res = layer(torch.randn(batch, length, 256, device="cuda", generator=g).half(), None, inference_params=params)
+    return (out, res, *params.key_value_memory_dict[0])
+
+
+FOUR = [(f, w) for f in ("mamba2", "mamba1") for w in ("w4", "w8")]
+
+
+@pytest.mark.parametrize("decode", [False, True])
+@pytest.mark.parametrize("family,weights", FOUR)
+def test_scales_in_half_precision_are_refused(family, weights, decode):
+    layer = _any_layer(family, weights).half()
+    with pytest.raises(RuntimeError, match="float32"):
+        _call(layer, 2, 1 if decode else 5, decode)
+
+
+@pytest.mark.parametrize("decode", [False, True])
+@pytest.mark.parametrize("part", ["in_proj", "conv1d", "scan", "out_proj", "norm"])
+@pytest.mark.parametrize("family,weights", FOUR)
+def test_a_part_left_on_the_cpu_is_refused(family, weights, part, decode):
+    layer = _any_layer(family, weights)
+    m = layer.mixer
+    scan = m.qchunk_scan if family == "mamba2" else m.selective_scan
+    {"scan": scan, "norm": layer.norm}.get(part, None if part in ("scan", "norm") else getattr(m, part, None)).cpu()
+    with pytest.raises(RuntimeError, match="CUDA"):
+        _call(layer, 2, 1 if decode else 5, decode)
+
+
+@pytest.mark.parametrize("family,weights", FOUR)
+def test_caches_elsewhere_than_the_input_are_filled_by_the_walk(family, weights):
+    layer = _any_layer(family, weights)
+    want = _call(layer, 2, 7, False)
+    conv, ssm = layer.allocate_inference_cache(2, 8)
+    got = _call(layer, 2, 7, False, (conv, ssm.cpu()))
+    tol = 0 if family == "mamba2" else 1                    # (the Mamba1 walk runs the sequence-last scan)
+    assert torch.equal(got[2], want[2]) and (got[3].int() - want[3].cpu().int()).abs().max() <= tol
