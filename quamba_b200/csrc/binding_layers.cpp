@@ -157,6 +157,11 @@ struct Lin {
         throw NotPlain{};
     }
   }
+  // has to_seqlen_last, the form a Mamba1 prefill multiplies with: one scale per side, whose places it swaps
+  bool seqlen_last() const {
+    const PyTypeObject* ty = Py_TYPE(m.self);
+    return ty == g_types.W4A8B8O8Linear || (ty == g_types.W8A8B8O8Linear && m.tensor(QBN_NAME(b)).numel() == 1);
+  }
   static Mod open(const Mod& parent, PyObject* name) { return parent.child(name, nullptr); }
 
   // the module's prepared weight, built or rebuilt by prepared() when a buffer was replaced or written in place
@@ -419,7 +424,7 @@ PyObject* mamba1_layer(const Args& a) {
             had_m = mx.child(QBN_NAME(had), g_types.QHadamard);
   const int64_t d = mx.integer(QBN_NAME(d_inner)), ds = mx.integer(QBN_NAME(d_state)), rank = mx.integer(QBN_NAME(dt_rank));
   if (in.k != dm || in.features != 2 * d || xp.k != d || xp.features != rank + 2 * ds || dtp.k != rank || dtp.features != d || dtp.n != d || outp.k != d ||
-      !in.int8 || !xp.int8 || !dtp.int8 || outp.int8 || ds != 16 || d % 16 != 0 || rank % 4 != 0)
+      !in.int8 || !xp.int8 || !dtp.int8 || outp.int8 || (!decode && (!in.seqlen_last() || !dtp.seqlen_last())) || ds != 16 || d % 16 != 0 || rank % 4 != 0)
     throw NotPlain{};
   const Tensor conv_st = a.opt_tensor(5), ssm_st = a.opt_tensor(6);
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };

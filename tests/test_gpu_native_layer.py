@@ -133,3 +133,26 @@ def test_caches_elsewhere_than_the_input_are_filled_by_the_walk(family, weights)
     got = _call(layer, 2, 7, False, (conv, ssm.cpu()))
     tol = 0 if family == "mamba2" else 1                    # (the Mamba1 walk runs the sequence-last scan)
     assert torch.equal(got[2], want[2]) and (got[3].int() - want[3].cpu().int()).abs().max() <= tol
+
+
+@pytest.mark.parametrize("weights", ["w8", "w4"])
+def test_mamba1_prefill_refuses_a_projection_without_the_sequence_last_form(weights):
+    """The parallel classes scale every column by itself and have no to_seqlen_last; a decode step takes them."""
+    from quamba_b200 import W4A8B8O8LinearParallel, W8A8B8O8LinearParallel
+    layer = _mamba1_layer(weights)
+    old = layer.mixer.in_proj
+    new = (W8A8B8O8LinearParallel if weights == "w8" else W4A8B8O8LinearParallel)(256, old.out_features, device="cuda")
+    new.weight = old.weight
+    if weights == "w8":
+        new.a, new.b = old.a, old.b * torch.linspace(0.5, 1.5, new.b.numel(), device="cuda")[None]
+    else:
+        new.s_channel, new.s_group, new.input_scale = old.s_channel, old.s_group, old.input_scale
+    layer.mixer.in_proj = new
+    with pytest.raises(TypeError if weights == "w4" else AttributeError):
+        _call(layer, 2, 5, False)
+    got = _call(layer, 3, 1, True)
+    hook = layer.mixer.conv1d.register_forward_hook(lambda *a: None)
+    want = _call(layer, 3, 1, True)
+    hook.remove()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
