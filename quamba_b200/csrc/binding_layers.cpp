@@ -433,7 +433,7 @@ PyObject* mamba1_layer(const Args& a) {
   if (cw.dim() != 2 || cw.size(0) != d || cw.size(1) != 4 || !cw.is_contiguous() || (cb.defined() && !cb.is_contiguous()) ||
       (conv_st.defined() && (conv_st.scalar_type() != at::kChar || !is(conv_st, {batch, d, 4}) || ssm_st.scalar_type() != at::kChar ||
                              !is(ssm_st, {batch, d, ds}) || !ssm_st.is_contiguous() || conv_st.device() != on || ssm_st.device() != on ||
-                             (conv_st.stride(1) == 1 && (conv_st.stride(0) % 4 != 0 || conv_st.stride(2) % 4 != 0)))))
+                             (conv_st.stride(1) == 1 && (conv_st.stride(0) % 4 != 0 || conv_st.stride(2) % 4 != 0 || reinterpret_cast<uintptr_t>(conv_st.data_ptr()) % 4 != 0)))))
     throw NotPlain{};
   const Tensor A = scan.tensor_on(QBN_NAME(A_log), at::kChar, on), D = scan.opt_tensor_on(QBN_NAME(D), at::kChar, on),
                bias = scan.opt_tensor_on(QBN_NAME(dt_bias), at::kChar, on);

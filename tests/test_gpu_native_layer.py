@@ -156,3 +156,19 @@ def test_mamba1_prefill_refuses_a_projection_without_the_sequence_last_form(weig
     hook.remove()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("decode", [False, True])
+@pytest.mark.parametrize("family,weights", FOUR)
+def test_caches_at_an_odd_address(family, weights, decode):
+    """Views of a caller's buffer that start on any byte, the conv cache with its channels innermost."""
+    layer = _any_layer(family, weights)
+    conv, ssm = layer.allocate_inference_cache(2, 8)
+    dim = conv.shape[1]
+    g = torch.Generator(device="cuda").manual_seed(1)
+    odd = lambda n: torch.randint(-90, 90, (n + 1,), device="cuda", generator=g).to(torch.int8)[1:]
+    c1, s1 = odd(2 * 4 * dim).view(2, 4, dim).transpose(1, 2), odd(ssm.numel()).view(ssm.shape)
+    c2, s2 = conv.copy_(c1), ssm.copy_(s1)
+    got, want = _call(layer, 2, 1 if decode else 6, decode, (c1, s1)), _call(layer, 2, 1 if decode else 6, decode, (c2, s2))
+    assert torch.equal(c1, c2) and (s1.int() - s2.int()).abs().max() <= 1          # (an unaligned state takes the plain update kernel)
+    assert (got[0].float() - want[0].float()).norm() <= 0.02 * want[0].float().norm()
