@@ -426,6 +426,8 @@ PyObject* mamba1_layer(const Args& a) {
   if (in.k != dm || in.features != 2 * d || xp.k != d || xp.features != rank + 2 * ds || dtp.k != rank || dtp.features != d || dtp.n != d || outp.k != d ||
       !in.int8 || !xp.int8 || !dtp.int8 || outp.int8 || (!decode && (!in.seqlen_last() || !dtp.seqlen_last())) || ds != 16 || d % 16 != 0 || rank % 4 != 0)
     throw NotPlain{};
+  // the channel-last scan counts a sequence's elements in 31 bits and the sequences in 16
+  if (!decode && (std::max({in.n, xp.n, d}) * len >= (int64_t(1) << 31) || batch >= 65536)) throw NotPlain{};
   const Tensor conv_st = a.opt_tensor(5), ssm_st = a.opt_tensor(6);
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
   const Tensor cw = conv.tensor_on(QBN_NAME(weight), at::kChar, on), cb = conv.opt_tensor_on(QBN_NAME(bias), at::kChar, on);

@@ -172,3 +172,17 @@ def test_caches_at_an_odd_address(family, weights, decode):
     got, want = _call(layer, 2, 1 if decode else 6, decode, (c1, s1)), _call(layer, 2, 1 if decode else 6, decode, (c2, s2))
     assert torch.equal(c1, c2) and (s1.int() - s2.int()).abs().max() <= 1          # (an unaligned state takes the plain update kernel)
     assert (got[0].float() - want[0].float()).norm() <= 0.02 * want[0].float().norm()
+
+
+def test_mamba1_sizes_beyond_the_channel_last_scan():
+    """It counts the elements of a sequence in 31 bits and the sequences in 16; the sequence-last kernel has no such limits."""
+    layer = _mamba1_layer("w8")
+    for shape in ((1, 1 << 21, 256), (65536, 1, 256)):
+        u = torch.empty(shape, dtype=torch.int8, device="cuda")
+        assert layer.mixer.native_layer(None, u, None, False, None) is None, shape
+    g = torch.Generator(device="cuda").manual_seed(4)
+    h = torch.randn(65537, 1, 256, device="cuda", generator=g).half()
+    for part in (slice(0, 64), slice(65500, 65537)):
+        want = layer(h[part], None)[0].float()
+        got = layer(h, None)[0][part].float()
+        assert (got - want).norm() <= 0.02 * want.norm()
