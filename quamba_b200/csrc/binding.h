@@ -164,6 +164,7 @@ struct Mod {
   // the sub-module, which must be exactly of class `type` and carry no hooks
   Mod child(PyObject* name, PyTypeObject* type) const;
   void require_plain(PyTypeObject* type) const;
+  void require_own(PyObject* method) const;                  // the method is the class's, not one set on the instance
 };
 
 struct Types {

@@ -50,6 +50,10 @@ void Mod::require_plain(PyTypeObject* type) const {
     throw NotPlain{};
 }
 
+void Mod::require_own(PyObject* method) const {
+  if (PyDict_GetItem(attrs, method) != nullptr) throw NotPlain{};
+}
+
 Mod Mod::child(PyObject* name, PyTypeObject* type) const {
   PyObject* mods = PyDict_GetItem(attrs, QBN_NAME(_modules));
   PyObject* c = mods != nullptr ? PyDict_GetItem(mods, name) : nullptr;
@@ -271,10 +275,9 @@ Tensor layer_output(const Tensor& out, int64_t batch, int64_t len, const Lin& li
 PyObject* mamba2_layer(const Args& a) {
   const Mod mx(a.object(1));
   const bool has_norm = !a.is_none(0), decode = a.flag(7);
-  if (has_norm) {
-    if (Py_TYPE(mx.self) != g_w4_mamba2 && Py_TYPE(mx.self) != g_w8_mamba2) throw NotPlain{};
-    mx.require_plain(nullptr);
-  }
+  if (Py_TYPE(mx.self) != g_w4_mamba2 && Py_TYPE(mx.self) != g_w8_mamba2) throw NotPlain{};   // a subclass may have a forward or step of its own
+  if (has_norm) mx.require_plain(nullptr);
+  if (decode) mx.require_own(QBN_NAME(step));
   if ((g_hooks != nullptr && PyDict_GET_SIZE(g_hooks) != 0) || (g_pre_hooks != nullptr && PyDict_GET_SIZE(g_pre_hooks) != 0)) throw NotPlain{};
   const Tensor x = a.tensor(2);
   if (!x.is_cuda() || x.dim() != 3 || !x.is_contiguous() || x.numel() == 0) throw NotPlain{};
@@ -284,6 +287,7 @@ PyObject* mamba2_layer(const Args& a) {
   const Lin in(mx, QBN_NAME(in_proj), on), outp(mx, QBN_NAME(out_proj), on);
   const Mod conv = mx.child(QBN_NAME(conv1d), g_types.Quamb2Conv1D), scan = mx.child(QBN_NAME(qchunk_scan), g_types.Quamba2ChunkScan),
             gn_m = mx.child(QBN_NAME(norm), g_types.QRMSNormGated), had_m = mx.child(QBN_NAME(had), g_types.QHadamard);
+  if (decode) { conv.require_own(QBN_NAME(update)); scan.require_own(QBN_NAME(update)); }
   const int64_t d = mx.integer(QBN_NAME(d_ssm)), groups = mx.integer(QBN_NAME(ngroups)), ds = mx.integer(QBN_NAME(d_state)),
                 nh = mx.integer(QBN_NAME(nheads)), hd = mx.integer(QBN_NAME(headdim)), gn = groups * ds, dim = d + 2 * gn;
   if (in.k != dm || !in.int8 || outp.int8 || outp.k != d || in.features != d + dim + nh || nh * hd != d) throw NotPlain{};
@@ -409,10 +413,9 @@ PyObject* mamba2_layer(const Args& a) {
 PyObject* mamba1_layer(const Args& a) {
   const Mod mx(a.object(1));
   const bool has_norm = !a.is_none(0), decode = a.flag(7);
-  if (has_norm) {
-    if (Py_TYPE(mx.self) != g_w4_mamba1 && Py_TYPE(mx.self) != g_w8_mamba1) throw NotPlain{};
-    mx.require_plain(nullptr);
-  }
+  if (Py_TYPE(mx.self) != g_w4_mamba1 && Py_TYPE(mx.self) != g_w8_mamba1) throw NotPlain{};   // a subclass may have a forward or step of its own
+  if (has_norm) mx.require_plain(nullptr);
+  if (decode) mx.require_own(QBN_NAME(step));
   if ((g_hooks != nullptr && PyDict_GET_SIZE(g_hooks) != 0) || (g_pre_hooks != nullptr && PyDict_GET_SIZE(g_pre_hooks) != 0)) throw NotPlain{};
   const Tensor x = a.tensor(2);
   if (!x.is_cuda() || x.dim() != 3 || !x.is_contiguous() || x.numel() == 0) throw NotPlain{};
@@ -422,6 +425,8 @@ PyObject* mamba1_layer(const Args& a) {
   const Lin in(mx, QBN_NAME(in_proj), on), xp(mx, QBN_NAME(x_proj), on), dtp(mx, QBN_NAME(dt_proj), on), outp(mx, QBN_NAME(out_proj), on);
   const Mod conv = mx.child(QBN_NAME(conv1d), g_types.QCausalConv1D), scan = mx.child(QBN_NAME(selective_scan), g_types.QSScan),
             had_m = mx.child(QBN_NAME(had), g_types.QHadamard);
+  if (decode) { conv.require_own(QBN_NAME(update)); scan.require_own(QBN_NAME(update)); }
+  else { in.m.require_own(QBN_NAME(to_seqlen_last)); dtp.m.require_own(QBN_NAME(to_seqlen_last)); }
   const int64_t d = mx.integer(QBN_NAME(d_inner)), ds = mx.integer(QBN_NAME(d_state)), rank = mx.integer(QBN_NAME(dt_rank));
   if (in.k != dm || in.features != 2 * d || xp.k != d || xp.features != rank + 2 * ds || dtp.k != rank || dtp.features != d || dtp.n != d || outp.k != d ||
       !in.int8 || !xp.int8 || !dtp.int8 || outp.int8 || (!decode && (!in.seqlen_last() || !dtp.seqlen_last())) || ds != 16 || d % 16 != 0 || rank % 4 != 0)

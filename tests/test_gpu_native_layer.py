@@ -186,3 +186,42 @@ def test_mamba1_sizes_beyond_the_channel_last_scan():
         want = layer(h[part], None)[0].float()
         got = layer(h, None)[0][part].float()
         assert (got - want).norm() <= 0.02 * want.norm()
+
+
+@pytest.mark.parametrize("through_block", [True, False])
+@pytest.mark.parametrize("family,weights", FOUR)
+def test_methods_of_a_subclass_or_an_instance_are_called(family, weights, through_block):
+    """What a user overrides, in a subclass of the mixer or on one module, runs in prefill and in decode."""
+    layer = _any_layer(family, weights)
+    m = layer.mixer
+    scan = m.qchunk_scan if family == "mamba2" else m.selective_scan
+    calls = []
+
+    def call(decode):
+        if through_block:
+            return _call(layer, 2, 1 if decode else 5, decode)
+        params = InferenceParams(max_seqlen=8, max_batch_size=2, seqlen_offset=int(decode))
+        return m(torch.ones(2, 1 if decode else 5, 256, dtype=torch.int8, device="cuda"), inference_params=params)
+
+    def watched(obj, name):
+        old = getattr(obj, name)
+        setattr(obj, name, lambda *a, **k: (calls.append(name), old(*a, **k))[1])
+
+    cases = [(m, "step", True), (m.conv1d, "update", True), (scan, "update", True)]
+    if family == "mamba1":
+        cases += [(m.in_proj, "to_seqlen_last", False), (m.dt_proj, "to_seqlen_last", False)]
+    for obj, name, decode in cases:
+        watched(obj, name)
+        call(decode)
+        assert calls == [name], (type(obj).__name__, name)
+        delattr(obj, name)
+        calls.clear()
+
+    class Mine(type(m)):
+        def step(self, *a):
+            calls.append("mine")
+            return super().step(*a)
+
+    m.__class__ = Mine
+    call(True)
+    assert calls == ["mine"]
