@@ -450,7 +450,7 @@ PyObject* norm_fwd(const Args& a) {
   const Tensor x = a.tensor(0), w = a.tensor(1), bias = a.opt_tensor(2), res = a.opt_tensor(4), slots = a.opt_tensor(8), own = a.opt_tensor(10);
   Tensor y = a.opt_tensor(11);
   if (slots.defined()) {
-    need(slots.dim() == 3 && slots.scalar_type() == at::kHalf && slots.stride(2) == 1 && slots.stride(1) == slots.size(2) && x.data_ptr() == slots.data_ptr(),
+    need(slots.dim() == 3 && slots.scalar_type() == at::kHalf && slots.select(0, 0).is_contiguous() && x.data_ptr() == slots.data_ptr(),
          "partials: fp16 (n, M, N) slots with contiguous rows, x = slots[0]");
     need(!own.defined() || (own.sizes() == x.sizes() && own.scalar_type() == at::kHalf && own.strides() == x.strides()),
          "partials: own piece must have the shape and strides of a slot");
