@@ -8,6 +8,7 @@ missing, importing this module raises.
 """
 import ctypes
 import re
+import threading
 from pathlib import Path
 
 _PKG = Path(__file__).resolve().parent
@@ -130,16 +131,16 @@ def set_call_trace(sink):
 
 class _Trace:
     def __init__(self, sink):
-        self.sink, self.start = sink, None
+        self.sink, self.pending = sink, threading.local()     # launches of several threads interleave
 
     def __call__(self, fn, phase, stream):
         import torch
         event = torch.cuda.Event(enable_timing=True)
         event.record(torch.cuda.ExternalStream(stream))
         if phase == 0:
-            self.start = event
+            self.pending.start = event
         else:
-            self.sink.append((fn, self.start, event))
+            self.sink.append((fn, self.pending.start, event))
 
 
 def call(fn: str, args, stream: int):

@@ -15,17 +15,24 @@ namespace qbn {
 
 PyObject* g_trace = nullptr;   // callable(entry point, 0 | 1, stream) around every launch, or null
 
-void run_call(const char* name, int (*f)(const void*, void*), const void* args, cudaStream_t st) {
-  if (g_trace != nullptr) call_trace(name, 0, st);
-  const int rc = f(args, st);
-  if (rc != QB_OK) throw std::runtime_error("quamba_b200 error " + std::to_string(rc) + ": " + qb_last_error());
-  if (g_trace != nullptr) call_trace(name, 1, st);
-}
-
-void call_trace(const char* name, int phase, cudaStream_t st) {
-  PyObject* r = PyObject_CallFunction(g_trace, "siK", name, phase, (unsigned long long)(uintptr_t)st);
+namespace {
+void call_trace(PyObject* trace, const char* name, int phase, cudaStream_t st) {
+  PyObject* r = PyObject_CallFunction(trace, "siK", name, phase, (unsigned long long)(uintptr_t)st);
   if (r == nullptr) throw PyErr{};
   Py_DECREF(r);
+}
+}  // namespace
+
+void run_call(const char* name, int (*f)(const void*, void*), const void* args, cudaStream_t st) {
+  const Ref trace = Ref::share(g_trace);
+  if (trace != nullptr) call_trace(trace, name, 0, st);
+  int rc;
+  {
+    const NoGil released;
+    rc = f(args, st);
+  }
+  if (rc != QB_OK) throw std::runtime_error("quamba_b200 error " + std::to_string(rc) + ": " + qb_last_error());
+  if (trace != nullptr) call_trace(trace, name, 1, st);
 }
 
 namespace {

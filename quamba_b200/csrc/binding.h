@@ -19,9 +19,29 @@ namespace qbn {
 using at::Tensor;
 
 struct PyErr {};                                             // a Python exception is already set
+// Python's other threads run while the library or the allocator works: a launch waits where the queue is full, and a first call
+// sets attributes or allocates.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+// A strong reference: between two launches other threads may replace what a module holds.
+class Ref {
+ public:
+  Ref() = default;
+  static Ref own(PyObject* o) { Ref r; r.o_ = o; return r; }
+  static Ref share(PyObject* o) { return own(Py_XNewRef(o)); }
+  Ref(const Ref& r) : o_(Py_XNewRef(r.o_)) {}
+  Ref(Ref&& r) noexcept : o_(r.o_) { r.o_ = nullptr; }
+  Ref& operator=(Ref r) noexcept { std::swap(o_, r.o_); return *this; }
+  ~Ref() { Py_XDECREF(o_); }
+  operator PyObject*() const { return o_; }
+
+ private:
+  PyObject* o_ = nullptr;
+};
 struct NotPlain {};                                          // the layer functions: walk the modules instead
 
-void call_trace(const char* name, int phase, cudaStream_t st);
 void run_call(const char* name, int (*f)(const void*, void*), const void* args, cudaStream_t st);
 #define QBN_CALL(fn, s, st) ::qbn::run_call(#fn, [](const void* qbn_p, void* qbn_st) { return fn(static_cast<const std::remove_reference_t<decltype(s)>*>(qbn_p), qbn_st); }, &(s), (st))
 
@@ -34,7 +54,11 @@ inline void cuda_i8(const Tensor& t, const char* name) {
 inline void cuda_f32(const Tensor& t, const char* name) {
   if (!t.is_cuda() || t.scalar_type() != at::kFloat) throw std::runtime_error(std::string(name) + " must be a float32 CUDA tensor");
 }
-inline Tensor contiguous(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+inline Tensor contiguous(const Tensor& t) {
+  if (t.is_contiguous()) return t;
+  const NoGil released;
+  return t.contiguous();
+}
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline int8_t* i8(const Tensor& t) { return static_cast<int8_t*>(ptr(t)); }
 inline float* f32(const Tensor& t) { return static_cast<float*>(ptr(t)); }
@@ -83,8 +107,12 @@ struct Device {
   cudaStream_t stream;
   c10::Device dev;
   explicit Device(const Tensor& t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.device().index()).stream()), dev(t.device()) {}
-  Tensor empty(at::IntArrayRef sizes, at::ScalarType t) const { return Tensor(at::detail::empty_cuda(sizes, t, dev, std::nullopt)); }
+  Tensor empty(at::IntArrayRef sizes, at::ScalarType t) const {
+    const NoGil released;
+    return Tensor(at::detail::empty_cuda(sizes, t, dev, std::nullopt));
+  }
   Tensor empty_strided(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType t) const {
+    const NoGil released;
     return Tensor(at::detail::empty_strided_cuda(sizes, strides, t, dev));
   }
 };
@@ -130,9 +158,7 @@ inline const Tensor& plain(const Tensor& t, at::ScalarType type, c10::Device dev
 
 // A torch.nn.Module as its dictionaries: plain attributes, buffers, sub-modules.
 struct Mod {
-  PyObject* self;
-  PyObject* attrs;
-  PyObject* buffers;
+  Ref self, attrs, buffers;
   explicit Mod(PyObject* o);
   PyObject* find(PyObject* name) const {                     // borrowed, null when absent
     PyObject* r = PyDict_GetItem(attrs, name);

@@ -32,11 +32,9 @@ PyObject* set_types(PyObject*, PyObject* dict) {
   Py_RETURN_NONE;
 }
 
-Mod::Mod(PyObject* o) : self(o) {
-  attrs = PyObject_GenericGetDict(o, nullptr);
+Mod::Mod(PyObject* o) : self(Ref::share(o)), attrs(Ref::own(PyObject_GenericGetDict(o, nullptr))) {
   if (attrs == nullptr) throw PyErr{};
-  Py_DECREF(attrs);                                          // the object keeps it alive
-  buffers = PyDict_GetItem(attrs, QBN_NAME(_buffers));
+  buffers = Ref::share(PyDict_GetItem(attrs, QBN_NAME(_buffers)));
   if (buffers == nullptr) throw NotPlain{};
 }
 
@@ -140,7 +138,9 @@ namespace {
 struct Lin {
   Mod m;
   int64_t k, n, features;
-  bool w4, int8;
+  bool w4, int8, has_alpha = false;
+  Tensor w, sa, sb;                                          // W8A8: weight and scales; W4A8: the input scale in sa
+  double alpha = 0.0;
   Lin(const Mod& parent, PyObject* name, c10::Device dev) : m(open(parent, name)) {
     const Types& t = g_types;
     PyTypeObject* ty = Py_TYPE(m.self);
@@ -153,9 +153,11 @@ struct Lin {
     if (w4) {
       if (m.integer(QBN_NAME(size_n)) != n || m.integer(QBN_NAME(size_k)) != k) throw NotPlain{};
       m.tensor_on(QBN_NAME(weight), at::kInt, dev);
-      m.tensor_on(QBN_NAME(input_scale), at::kFloat, dev);
+      sa = m.tensor_on(QBN_NAME(input_scale), at::kFloat, dev);
     } else {
-      const Tensor w = m.tensor_on(QBN_NAME(weight), at::kChar, dev), sa = m.tensor_on(QBN_NAME(a), at::kFloat, dev), sb = m.tensor_on(QBN_NAME(b), at::kFloat, dev);
+      w = m.tensor_on(QBN_NAME(weight), at::kChar, dev); sa = m.tensor_on(QBN_NAME(a), at::kFloat, dev); sb = m.tensor_on(QBN_NAME(b), at::kFloat, dev);
+      has_alpha = ty != t.W8A8B8O8LinearParallel;
+      if (has_alpha) alpha = m.num(QBN_NAME(alpha));
       if (w.dim() != 2 || w.size(0) != k || w.size(1) != n || w.stride(0) != 1 || w.stride(1) % 16 != 0 || !sa.is_contiguous() || !sb.is_contiguous() ||
           sa.numel() != 1 || (sb.numel() != 1 && sb.numel() != n))
         throw NotPlain{};
@@ -164,13 +166,13 @@ struct Lin {
   // has to_seqlen_last, the form a Mamba1 prefill multiplies with: one scale per side, whose places it swaps
   bool seqlen_last() const {
     const PyTypeObject* ty = Py_TYPE(m.self);
-    return ty == g_types.W4A8B8O8Linear || (ty == g_types.W8A8B8O8Linear && m.tensor(QBN_NAME(b)).numel() == 1);
+    return ty == g_types.W4A8B8O8Linear || (ty == g_types.W8A8B8O8Linear && sb.numel() == 1);
   }
   static Mod open(const Mod& parent, PyObject* name) { return parent.child(name, nullptr); }
 
   // the module's prepared weight, built or rebuilt by prepared() when a buffer was replaced or written in place
-  PyObject* prepared() const {
-    PyObject* p = PyDict_GetItem(m.attrs, QBN_NAME(_prep));
+  Ref prepared() const {
+    const Ref p = Ref::share(PyDict_GetItem(m.attrs, QBN_NAME(_prep)));
     if (p != nullptr && p != Py_None) {
       PyObject* d = attrs_of(p);
       PyObject* src = item(d, QBN_NAME(_src));
@@ -183,29 +185,28 @@ struct Lin {
       }
       if (fresh) return p;
     }
-    PyObject* q = PyObject_CallMethodNoArgs(m.self, QBN_NAME(prepared));
+    const Ref q = Ref::own(PyObject_CallMethodNoArgs(m.self, QBN_NAME(prepared)));
     if (q == nullptr) throw PyErr{};
-    Py_DECREF(q);                                            // the module keeps it
     return q;
   }
 
   // as_matrix: the matrix form even for one row, with the two scales applied in the order of to_seqlen_last
   void run(const int8_t* a, int64_t lda, int64_t rows, void* out, int64_t ldo, cudaStream_t st, bool as_matrix = false) const {
     if (w4) {
-      PyObject* p = prepared();
+      const Ref p = prepared();
       const W4Dims d = w4_dims(p);
-      w4a8_run(p, d, a, lda, rows, f32(m.tensor(QBN_NAME(input_scale))), false, out, ldo, int8, false, st);
+      need(d.n == n && d.k == k, "the weight was replaced by one of another shape during the call");
+      w4a8_run(p, d, a, lda, rows, f32(sa), false, out, ldo, int8, false, st);
       return;
     }
-    const Tensor w = m.tensor(QBN_NAME(weight)), sa = m.tensor(QBN_NAME(a)), sb = m.tensor(QBN_NAME(b));
     qb_w8a8_gemm_args s{};
     s.a = a; s.b = i8(w); s.out = out; s.a_row_stride = lda; s.b_col_stride = w.stride(1); s.out_row_stride = ldo;
     s.m = rows; s.n = n; s.k = k; s.out_dtype = int8 ? 0 : 1;
     if (as_matrix) {
       s.a_scale = f32(sb); s.b_scale = f32(sa);
-    } else if (rows == 1 && Py_TYPE(m.self) != g_types.W8A8B8O8LinearParallel) {
+    } else if (rows == 1 && has_alpha) {
       s.use_alpha = 1;
-      s.alpha = m.num(QBN_NAME(alpha));
+      s.alpha = alpha;
     } else {
       s.a_scale = f32(sa); s.b_scale = f32(sb); s.b_scale_per_col = sb.numel() != 1;
       s.round_half_away = rows == 1;
@@ -336,6 +337,10 @@ PyObject* mamba2_layer(const Args& a) {
     throw NotPlain{};
   PyObject* lim = scan.get(QBN_NAME(dt_limit));
   if (!PyTuple_Check(lim) || PyTuple_GET_SIZE(lim) != 2) throw NotPlain{};
+  const double dt_min = as_double(PyTuple_GET_ITEM(lim, 0)), dt_max = std::min(as_double(PyTuple_GET_ITEM(lim, 1)), 3.0e38);
+  const bool softplus = scan.flag(QBN_NAME(delta_softplus)), before_gate = gn_m.flag(QBN_NAME(norm_before_gate));
+  const int64_t chunk = scan.integer(QBN_NAME(chunk_size));
+  const double g_eps = gn_m.num(QBN_NAME(eps)), g_z = gn_m.num(QBN_NAME(z_scale));
   const Rotation had(had_m);
   if (had.blocks <= 0 || d % had.blocks != 0) throw NotPlain{};
 
@@ -361,7 +366,7 @@ PyObject* mamba2_layer(const Args& a) {
     s.x_scales = f32(xs); s.dt_scale = f32(dts); s.A_scale = f32(As); s.B_scale = f32(Bs); s.C_scale = f32(Cs); s.D_scale = f32(Ds);
     s.head_group_range = i32(hgr); s.dim_group_range = i32(dgr); s.out = y.data_ptr();
     s.batch = batch; s.nheads = nh; s.headdim = hd; s.ngroups = groups; s.dstate = ds; s.grouped = grouped;
-    s.nhead_groups = grouped ? hgr.size(1) : 0; s.ndim_groups = grouped ? dgr.size(2) : 0; s.dt_softplus = scan.flag(QBN_NAME(delta_softplus));
+    s.nhead_groups = grouped ? hgr.size(1) : 0; s.ndim_groups = grouped ? dgr.size(2) : 0; s.dt_softplus = softplus;
   };
   if (decode) {
     qb_quamba2_conv1d_update_args s = c.update_args(dim);
@@ -384,21 +389,21 @@ PyObject* mamba2_layer(const Args& a) {
     QBN_CALL(qb_quamba2_conv1d_fwd, s, st);
     qb_ssd_args t{};
     scan_common(t);
-    const int64_t chunk = scan.integer(QBN_NAME(chunk_size)), wsb = qb_ssd_workspace_bytes(batch, len, nh, hd, groups, ds, chunk);
+    const int64_t wsb = qb_ssd_workspace_bytes(batch, len, nh, hd, groups, ds, chunk);
     need(wsb > 0, "invalid SSD shape");
     const Tensor ws = dev.empty({wsb}, at::kByte);
     const Tensor fin = ssm_st.defined() ? ssm_st : dev.empty({batch, nh, hd, ds}, at::kChar);
     t.ssm_state_scale = f32(ss); t.final_states = i8(fin); t.workspace = ws.data_ptr(); t.workspace_bytes = wsb;
     t.x_sb = len * d; t.x_sl = d; t.x_sh = hd; t.dt_sb = len * in.n; t.dt_sl = in.n; t.B_sb = t.C_sb = len * gn; t.B_sl = t.C_sl = gn; t.B_sg = t.C_sg = ds;
     t.seqlen = len; t.chunk_size = chunk; t.D_has_hdim = D.defined() && hdim;
-    t.dt_min = as_double(PyTuple_GET_ITEM(lim, 0)); t.dt_max = std::min(as_double(PyTuple_GET_ITEM(lim, 1)), 3.0e38);
+    t.dt_min = dt_min; t.dt_max = dt_max;
     QBN_CALL(qb_ssd_chunk_scan_fwd, t, st);
   }
   const Tensor g = dev.empty({rows, d}, at::kHalf);
   qb_rmsnorm_args s{};
   s.x = y.data_ptr(); s.weight = gw.data_ptr(); s.z = z; s.out = g.data_ptr(); s.x_row_stride = s.out_row_stride = d; s.z_row_stride = in.n;
-  s.rows = rows; s.group_size = gsize; s.ngroups = d / gsize; s.out_kind = 2; s.norm_before_gate = gn_m.flag(QBN_NAME(norm_before_gate)); s.is_rms_norm = 1;
-  s.eps = gn_m.num(QBN_NAME(eps)); s.z_scale = gn_m.num(QBN_NAME(z_scale));
+  s.rows = rows; s.group_size = gsize; s.ngroups = d / gsize; s.out_kind = 2; s.norm_before_gate = before_gate; s.is_rms_norm = 1;
+  s.eps = g_eps; s.z_scale = g_z;
   QBN_CALL(qb_rmsnorm_gated, s, st);
   const Tensor q = dev.empty({rows, d}, at::kChar);
   had.run(g, q, rows, d, st);
@@ -455,6 +460,9 @@ PyObject* mamba1_layer(const Args& a) {
   if (!is(A, {d, ds}) || !A.is_contiguous() || (D.defined() && (D.numel() != d || !D.is_contiguous())) ||
       (bias.defined() && (bias.numel() != d || !bias.is_contiguous())))
     throw NotPlain{};
+  const double c_in = conv.num(QBN_NAME(input_scale)), c_w = conv.num(QBN_NAME(weight_scale)), c_out = conv.num(QBN_NAME(output_scale)),
+               c_b = conv.num(QBN_NAME(bias_scale));
+  const bool softplus = scan.flag(QBN_NAME(delta_softplus));
   const Rotation had(had_m);
   if (had.blocks <= 0 || d % had.blocks != 0) throw NotPlain{};
 
@@ -474,8 +482,7 @@ PyObject* mamba1_layer(const Args& a) {
   int8_t* z = i8(xz) + d;
   auto conv_common = [&](auto& s) {
     s.x = i8(xz); s.out = i8(cx); s.weight = i8(cw); s.bias = i8(cb); s.batch = batch; s.dim = d; s.width = 4; s.x_sd = 1; s.out_sd = 1; s.silu = 1;
-    s.scale_x = conv.num(QBN_NAME(input_scale)); s.scale_w = conv.num(QBN_NAME(weight_scale)); s.scale_out = conv.num(QBN_NAME(output_scale));
-    s.scale_b = conv.num(QBN_NAME(bias_scale));
+    s.scale_x = c_in; s.scale_w = c_w; s.scale_out = c_out; s.scale_b = c_b;
     if (conv_st.defined()) { s.conv_state = i8(conv_st); s.state_sb = conv_st.stride(0); s.state_sd = conv_st.stride(1); s.state_sw = conv_st.stride(2); }
   };
   if (decode) {
@@ -499,7 +506,7 @@ PyObject* mamba1_layer(const Args& a) {
     t.z_scale = f32(zs); t.dt_bias_scale = f32(bs); t.out = y.data_ptr();
     t.state_sb = d * ds; t.state_sh = d * ds; t.state_sp = ds; t.x_sb = t.x_sh = d; t.dt_sb = t.dt_sh = d; t.dt_sp = 1; t.A_sh = d * ds; t.A_sp = ds; t.A_sn = 1;
     t.B_sb = t.B_sg = t.C_sb = t.C_sg = xp.n; t.D_sh = d; t.D_sp = 1; t.z_sb = t.z_sh = in.n; t.bias_sh = d; t.bias_sp = 1; t.out_sb = t.out_sh = d;
-    t.batch = batch; t.nheads = 1; t.headdim = d; t.dstate = ds; t.ngroups = 1; t.dt_softplus = scan.flag(QBN_NAME(delta_softplus));
+    t.batch = batch; t.nheads = 1; t.headdim = d; t.dstate = ds; t.ngroups = 1; t.dt_softplus = softplus;
     QBN_CALL(qb_sscan_update, t, st);
   } else {
     qb_sscan_fwd_args t{};
@@ -508,7 +515,7 @@ PyObject* mamba1_layer(const Args& a) {
     t.delta_bias_scale = f32(bs); t.ssm_state_scale = f32(ss); t.out = y.data_ptr();
     t.u_sb = t.delta_sb = len * d; t.u_sl = t.delta_sl = d; t.u_sd = t.delta_sd = t.z_sd = 1; t.z_sb = len * in.n; t.z_sl = in.n;
     t.B_sb = t.C_sb = len * xp.n; t.B_sl = t.C_sl = xp.n; t.B_sn = t.C_sn = 1;
-    t.batch = batch; t.dim = d; t.seqlen = len; t.dstate = ds; t.n_groups = 1; t.delta_softplus = scan.flag(QBN_NAME(delta_softplus));
+    t.batch = batch; t.dim = d; t.seqlen = len; t.dstate = ds; t.n_groups = 1; t.delta_softplus = softplus;
     t.channel_last = 1;
     t.final_state = ssm_st.defined() ? i8(ssm_st) : nullptr;
     t.workspace_bytes = qb_sscan_fwd_workspace_bytes(batch, d);

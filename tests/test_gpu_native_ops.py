@@ -16,3 +16,45 @@ def test_partial_slots_of_one_row():
     w = torch.ones(256, device="cuda", dtype=torch.float16)
     call = lambda s: ops._qlayer_norm_fwd(s[0], w, None, 1e-5, static_out_scale=0.05, is_rms_norm=True, partials=(s, -1, None))[0]
     assert torch.equal(call(slots), call(slots.contiguous()))
+
+
+@pytest.mark.parametrize("level", ["operator", "layer"])
+def test_other_python_threads_run_while_a_launch_waits(level):
+    """Behind a kernel of about half a second the launch queue fills up and a launch waits for room; another thread of the process,
+    which only looks at the clock, goes on meanwhile."""
+    import threading
+    import time
+    if level == "operator":
+        x = torch.zeros(1, 256, device="cuda", dtype=torch.int8)
+        st, w = torch.zeros(1, 256, 4, device="cuda", dtype=torch.int8), torch.zeros(256, 4, device="cuda", dtype=torch.int8)
+        call = lambda: ops.quant_causal_conv1d_cuda.update(x, st, 0.1, w, 0.1, 0.1, 0.1, None, True)
+        calls = 4000
+    else:
+        from quamba_b200 import InferenceParams
+        from test_gpu_native_layer import _layer
+        m = _layer("w4", False).mixer
+        u, params = torch.zeros(1, 1, 256, device="cuda", dtype=torch.int8), InferenceParams(max_seqlen=8, max_batch_size=1, seqlen_offset=1)
+        call = lambda: m.native_layer(None, u, None, False, params)
+        calls = 1000
+    call()
+    torch.cuda.synchronize()
+    gap, stop = [0.0], threading.Event()
+
+    def watch():
+        last = time.perf_counter()
+        while not stop.is_set():
+            now = time.perf_counter()
+            gap[0], last = max(gap[0], now - last), now
+            time.sleep(0.001)
+
+    t = threading.Thread(target=watch)
+    t.start()
+    t0 = time.perf_counter()
+    torch.cuda._sleep(1_000_000_000)
+    for _ in range(calls):
+        call()
+    torch.cuda.synchronize()
+    took = time.perf_counter() - t0
+    stop.set()
+    t.join()
+    assert took > 0.4 and gap[0] < 0.15, (took, gap[0])
