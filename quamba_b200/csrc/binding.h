@@ -2,6 +2,7 @@
 #pragma once
 
 #include <Python.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -138,8 +139,8 @@ PyObject* entry(PyObject*, PyObject* const* v, Py_ssize_t n) {
   } catch (const PyErr&) {
   } catch (const NotPlain&) {
     Py_RETURN_NONE;
-  } catch (const c10::Error& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+  } catch (const c10::Error&) {
+    torch::translate_exception_to_python(std::current_exception());   // torch's own types: out of memory, index, value errors
   } catch (const std::exception& e) {
     PyErr_SetString(PyExc_RuntimeError, e.what());
   }

@@ -58,3 +58,12 @@ def test_other_python_threads_run_while_a_launch_waits(level):
     stop.set()
     t.join()
     assert took > 0.4 and gap[0] < 0.15, (took, gap[0])
+
+
+def test_errors_keep_their_python_types():
+    """An output that does not fit raises torch's out-of-memory error, which callers catch to retry with less."""
+    x = torch.zeros(1, 256, device="cuda", dtype=torch.float16).expand(1 << 36, 256)     # 16 TB of int8 asked for
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.quant_hadamard.fast_hadamard_transform(x, 1.0)
+    y = torch.zeros(2, 256, device="cuda", dtype=torch.float16)
+    assert ops.quant_hadamard.fast_hadamard_transform(y, 1.0).shape == y.shape
