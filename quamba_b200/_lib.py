@@ -94,7 +94,11 @@ def native():
         try:
             from . import _native as mod
         except ImportError as e:
-            raise RuntimeError(f"quamba_b200/_native.so cannot be loaded ({e}): build it with `python -m quamba_b200.build`") from e
+            raise RuntimeError(f"quamba_b200/_native cannot be loaded ({e}): build it with `python -m quamba_b200.build`") from e
+        import torch
+        if mod.torch_version != torch.__version__:            # it is compiled against torch's C++ classes
+            raise RuntimeError(f"quamba_b200/_native was built for torch {mod.torch_version}, this is {torch.__version__}: build it with "
+                               "`python -m quamba_b200.build`")
         from .modules import plain_types
         mod.set_types(plain_types())
         _native = mod

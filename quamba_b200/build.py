@@ -1,9 +1,12 @@
 """Builds the two native libraries in-tree (no JIT cache, no torch extension machinery):
 
-    libquamba_b200.so   the kernels behind the C ABI, nvcc for sm_100a
-    _native.so          the host path (CPython extension over torch's C++ API), g++
+    libquamba_b200.so    the kernels behind the C ABI, nvcc for sm_100a
+    _native.<tag>.so     the host path (CPython extension over torch's C++ API), g++; the tag is the interpreter's
 
     python -m quamba_b200.build            # rebuilds what is out of date
+
+An object is out of date when a file it is made of is newer, or when the command that would make it is not the one that did: the
+host path's names the interpreter's and torch's headers and torch's version.
 """
 import os
 import subprocess
@@ -14,7 +17,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libquamba_b200.so"
-NATIVE = PKG / "_native.so"
+NATIVE = PKG / ("_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["lib.cu", "conv1d.cu", "hadamard.cu", "hadamard_tc.cu", "sscan.cu", "sscan_cl.cu", "ssd.cu", "ssd_tc.cu", "linear.cu", "gemm_tc.cu", "norm.cu",
            "embedding.cu", "decode.cu", "peer.cu"]
 NATIVE_SOURCES = ["binding.cpp", "binding_layers.cpp"]
@@ -23,8 +26,12 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17",
 CUDA = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 
 
-def _stale(obj: Path, src: Path) -> bool:
-    if not obj.exists():
+def _command_file(obj: Path) -> Path:
+    return obj.with_suffix(".cmd")
+
+
+def _stale(obj: Path, src: Path, cmd) -> bool:
+    if not obj.exists() or not _command_file(obj).exists() or _command_file(obj).read_text() != " ".join(cmd):
         return True
     t = obj.stat().st_mtime
     headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.inc")) if src.suffix == ".cu" else list(CSRC.glob("*.h"))
@@ -39,7 +46,7 @@ def _native_flags():
     import torch
     inc = Path(torch.__file__).parent / "include"
     dirs = [inc, inc / "torch" / "csrc" / "api" / "include", CUDA / "include", sysconfig.get_paths()["include"]]
-    return ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    return ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f'-DQBN_TORCH_VERSION="{torch.__version__}"', f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
             *[f for d in dirs for f in ("-isystem", str(d))]], Path(torch.__file__).parent / "lib"
 
 
@@ -52,12 +59,15 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     procs = []
     for name in SOURCES + NATIVE_SOURCES:
         src, obj = CSRC / name, objdir / (name + ".o")
-        if force or _stale(obj, src):
-            cmd = [nvcc, *NVCC_FLAGS] if src.suffix == ".cu" else [cxx, *flags]
-            procs.append((name, subprocess.Popen([*cmd, "-c", str(src), "-o", str(obj)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+        cmd = [nvcc, *NVCC_FLAGS] if src.suffix == ".cu" else [cxx, *flags]
+        if force or _stale(obj, src, cmd):
+            _command_file(obj).unlink(missing_ok=True)
+            procs.append((name, cmd, subprocess.Popen([*cmd, "-c", str(src), "-o", str(obj)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
-    for name, p in procs:
+    for name, cmd, p in procs:
         out, _ = p.communicate()
+        if p.returncode == 0:
+            _command_file(objdir / (name + ".o")).write_text(" ".join(cmd))
         if verbose or p.returncode != 0:
             sys.stderr.write(f"--- {name} ---\n{out}\n")
         (objdir / (name + ".log")).write_text(out)
@@ -67,6 +77,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     kernels, native = ([str(objdir / (n + ".o")) for n in names] for names in (SOURCES, NATIVE_SOURCES))
     if _older(LIB, kernels):
         subprocess.run([nvcc, "-shared", "-o", str(LIB), *kernels, "-gencode", "arch=compute_100a,code=sm_100a"], check=True)
+    (PKG / "_native.so").unlink(missing_ok=True)             # an untagged one would be loaded by any interpreter
     if _older(NATIVE, native):
         subprocess.run([cxx, "-shared", "-o", str(NATIVE), *native, f"-L{PKG}", "-l:libquamba_b200.so",
                         f"-L{torch_lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"],

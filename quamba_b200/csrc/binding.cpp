@@ -542,4 +542,11 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Host path of quamba_b2
 }  // namespace
 }  // namespace qbn
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&qbn::kModule); }
+PyMODINIT_FUNC PyInit__native() {
+  PyObject* m = PyModule_Create(&qbn::kModule);
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", QBN_TORCH_VERSION) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}
