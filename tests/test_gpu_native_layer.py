@@ -225,3 +225,27 @@ def test_methods_of_a_subclass_or_an_instance_are_called(family, weights, throug
     m.__class__ = Mine
     call(True)
     assert calls == ["mine"]
+
+
+@pytest.mark.parametrize("weights", ["w8", "w4"])
+@pytest.mark.parametrize("batch", [1, 2, 9, 16, 40])
+def test_mamba1_decode_against_the_module_walk(weights, batch):
+    """The same operators on strided views instead of copies: the integer products are equal, the state update may take another
+    kernel for the alignment of B and C."""
+    layer = _mamba1_layer(weights)
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    outs = []
+    for native in (True, False):
+        hook = None if native else layer.mixer.conv1d.register_forward_hook(lambda *a: None)
+        conv, ssm = layer.allocate_inference_cache(batch, 8)
+        g.manual_seed(batch)
+        conv.copy_(torch.randint(-100, 100, conv.shape, device="cuda", generator=g))
+        ssm.copy_(torch.randint(-100, 100, ssm.shape, device="cuda", generator=g))
+        outs.append(_call(layer, batch, 1, True, (conv, ssm)))
+        if hook is not None:
+            hook.remove()
+    (ya, ra, ca, sa), (yb, rb, cb, sb) = outs
+    assert torch.equal(ra, rb) and torch.equal(ca, cb)
+    diff = (sa.int() - sb.int()).abs()
+    assert diff.max() <= 1 and (diff != 0).float().mean() <= 2e-3
+    assert (ya.float() - yb.float()).norm() <= 0.02 * yb.float().norm()
