@@ -290,7 +290,7 @@ def run_head_parallel(args, rank, local_rank, world, pk):
                 "d2h_bytes_per_step": bp.BATCH * bp.CFG8B["vocab_size"] * 2,
                 "note": "every rank copies the token ids from pinned host memory and its last-token logits back to pinned host memory inside the timed region"},
         "gpu_launches": args.steps * r["layers"] * (bp.BATCH // r["chunk_sequences"]) * 8,
-        "roofline": {"kernel": "gemm_s8_tcgen05 (in_proj + out_proj shards)", "bound": "tensor", "achieved": r["gemm_tops_per_gpu"], "peak": pk["i8"],
+        "roofline": {"kernel": "gemm_s8_kernel (in_proj + out_proj shards)", "bound": "tensor", "achieved": r["gemm_tops_per_gpu"], "peak": pk["i8"],
                      "unit": "TOP/s", "frac": r["gemm_tops_per_gpu"] / pk["i8"], "traffic": None, "peak_source": pk["i8_source"],
                      "note": "GEMM flops of the step per GPU over the compute-only step time (all kernels, no collective)"},
     }
@@ -390,7 +390,7 @@ def run_ours(args, rank, local_rank, world):
     if top in ("qb_w4a8_gemm", "qb_w8a8_gemm"):
         achieved = m["n_layer"] * gemm_flops_layer / (top_ms * 1e-3) / 1e12
         traffic, traffic_source = gemm_traffic()
-        roof = {"kernel": "gemm_s8_tcgen05 (in_proj + out_proj of 64 layers)", "bound": "tensor", "achieved": achieved, "peak": pk["i8"],
+        roof = {"kernel": "gemm_s8_kernel (in_proj + out_proj of 64 layers)", "bound": "tensor", "achieved": achieved, "peak": pk["i8"],
                 "unit": "TOP/s", "frac": achieved / pk["i8"], "traffic": traffic, "traffic_source": traffic_source, "peak_source": pk["i8_source"],
                 "algorithmic_flops": m["n_layer"] * gemm_flops_layer, "ms": top_ms}
     else:

@@ -172,7 +172,7 @@ def op_ssd_update(dev, gen, ops):
         return lambda: ops.quant_sscan_update_triton(d["st"], d["x"], s(0.03), d["dt"], s(0.03), A, s(0.02), s(0.01), d["Bm"],
                                                      s(0.03), d["Cm"], s(0.03), Dv, s(0.01), None, None, bias, None, True)
     return dict(workload=f"Mamba2 int8 state update (decode) B{B} H{H} P{P} N{N}", bytes=by, flops=0, nsets=n, make=mk,
-                kernel="sscan_update_kernel", launches=1)
+                kernel="sscan_update_warp_kernel", launches=1)
 
 
 def _w4a8(dev, gen, ops, M, K, N, out_int8, tag, group=128):
@@ -196,8 +196,7 @@ def _w4a8(dev, gen, ops, M, K, N, out_int8, tag, group=128):
         return lambda: fn(xs[i], packs[i % len(packs)], st, sc, sg, ws, M, N, K, False)
     return dict(workload=f"W4A8 GEMM {tag}: M{M} K{K} N{N}, int4 {'group-128' if group > 0 else 'per-channel'} weights, {'int8' if out_int8 else 'fp16'} out",
                 bytes=by, flops=2 * M * N * K, nsets=n, make=mk, launches=1,
-                kernel=("gemm_s8_tcgen05_persistent_kernel" if M >= 128 else "gemm_s8_tcgen05_kernel<64>" if M >= 32 else
-                        "gemv_s4_kernel" if group < 0 else "gemv_s8_kernel"),
+                kernel="gemm_s8_kernel" if M > 8 else "gemv_s4_kernel" if group < 0 else "gemv_s8_kernel",
                 note="weights unpacked to int8 once at first use (cached); the timed GEMM streams int8 weights")
 
 
@@ -228,7 +227,7 @@ def op_rmsnorm(dev, gen, ops):
     def mk(i):
         return lambda: ops._qlayer_norm_fwd(xs[i], w, None, 1e-5, rs[i], static_out_scale=0.03, is_rms_norm=True)
     return dict(workload=f"QRMSNorm + residual add, Mamba2-2.7B block norm at 1 x 2048 tokens: M{M} N{N}, fp16 x, fp32 residual in and out, int8 out",
-                bytes=by, flops=0, nsets=n, make=mk, kernel="norm_quant_kernel<2, 0, 5>", launches=1)
+                bytes=by, flops=0, nsets=n, make=mk, kernel="norm_quant_kernel", launches=1)
 
 
 def op_rmsnorm_partials(dev, gen, ops):
@@ -245,7 +244,7 @@ def op_rmsnorm_partials(dev, gen, ops):
                                             partials=(xs[i], 0, None))
     return dict(workload=f"QRMSNorm + residual add over the sum of {T} partial inputs (head-parallel Mamba2-8B at eight ranks, one chunk's rows "
                          f"of one rank): M{M} N{N}, {T} fp16 slots, fp32 residual in and out, int8 out",
-                bytes=by, flops=0, nsets=n, make=mk, kernel="norm_quant_kernel<4, 0, 4> (n_partials = 8)", launches=1)
+                bytes=by, flops=0, nsets=n, make=mk, kernel="norm_quant_kernel (n_partials = 8)", launches=1)
 
 
 def op_rmsnorm_gated(dev, gen, ops):
@@ -260,7 +259,7 @@ def op_rmsnorm_gated(dev, gen, ops):
         return lambda: ops._qlayer_normgated_fwd(xs[i], w, None, 1e-5, q_z=zs[i], z_scale=0.02, use_float16_output=True,
                                                  group_size=N, norm_before_gate=False, is_rms_norm=True)
     return dict(workload=f"gated RMSNorm, Mamba2-2.7B at 1 x 2048 tokens: M{M} N{N}, fp16 x, int8 gate, fp16 out",
-                bytes=by, flops=0, nsets=n, make=mk, kernel="norm_quant_kernel<4, 1, 5>", launches=1)
+                bytes=by, flops=0, nsets=n, make=mk, kernel="norm_quant_kernel (gated)", launches=1)
 
 
 def op_w4a8_decode(dev, gen, ops):
@@ -370,7 +369,7 @@ def op_w8a8(dev, gen, ops):
     def mk(i):
         return lambda: ops.quant_linear_cuda.cutlass_scaled_mm_dq(ys[i], xs[i], w, a, b)
     return dict(workload=f"W8A8 GEMM Mamba1-2.8B in_proj, 16 x 1024 tokens: M{M} K{K} N{N}, int8 out", bytes=by,
-                flops=2 * M * N * K, nsets=n, make=mk, kernel="gemm_s8_tcgen05_kernel", launches=1)
+                flops=2 * M * N * K, nsets=n, make=mk, kernel="gemm_s8_kernel", launches=1)
 
 
 OPS = {"conv": op_conv, "conv_update": op_conv_update, "hadamard": op_hadamard, "sscan": op_sscan, "ssd": op_ssd,
