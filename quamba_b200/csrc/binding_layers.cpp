@@ -138,9 +138,9 @@ namespace {
 struct Lin {
   Mod m;
   int64_t k, n, features;
-  bool w4, int8, has_alpha = false;
+  bool w4, int8;
   Tensor w, sa, sb;                                          // W8A8: weight and scales; W4A8: the input scale in sa
-  double alpha = 0.0;
+  Ref alpha;                                                 // W8A8 with one scale per side: what a single row is scaled by
   Lin(const Mod& parent, PyObject* name, c10::Device dev) : m(open(parent, name)) {
     const Types& t = g_types;
     PyTypeObject* ty = Py_TYPE(m.self);
@@ -156,8 +156,7 @@ struct Lin {
       sa = m.tensor_on(QBN_NAME(input_scale), at::kFloat, dev);
     } else {
       w = m.tensor_on(QBN_NAME(weight), at::kChar, dev); sa = m.tensor_on(QBN_NAME(a), at::kFloat, dev); sb = m.tensor_on(QBN_NAME(b), at::kFloat, dev);
-      has_alpha = ty != t.W8A8B8O8LinearParallel;
-      if (has_alpha) alpha = m.num(QBN_NAME(alpha));
+      if (ty != t.W8A8B8O8LinearParallel) alpha = Ref::share(m.get(QBN_NAME(alpha)));
       if (w.dim() != 2 || w.size(0) != k || w.size(1) != n || w.stride(0) != 1 || w.stride(1) % 16 != 0 || !sa.is_contiguous() || !sb.is_contiguous() ||
           sa.numel() != 1 || (sb.numel() != 1 && sb.numel() != n))
         throw NotPlain{};
@@ -204,9 +203,9 @@ struct Lin {
     s.m = rows; s.n = n; s.k = k; s.out_dtype = int8 ? 0 : 1;
     if (as_matrix) {
       s.a_scale = f32(sb); s.b_scale = f32(sa);
-    } else if (rows == 1 && has_alpha) {
+    } else if (rows == 1 && alpha != nullptr) {
       s.use_alpha = 1;
-      s.alpha = alpha;
+      s.alpha = as_double(alpha);
     } else {
       s.a_scale = f32(sa); s.b_scale = f32(sb); s.b_scale_per_col = sb.numel() != 1;
       s.round_half_away = rows == 1;

@@ -134,3 +134,15 @@ def allclose_report(a, b, rtol, atol):
     tol = atol + rtol * b.abs()
     bad = err > tol
     return bool(not bad.any()), f"max err {err.max().item():.4g}, violations {int(bad.sum())}/{bad.numel()}, ref max {b.abs().max().item():.4g}"
+
+
+def launched(fn, part):
+    """Does ``fn`` launch a kernel with ``part`` in its name?  True as well where the profiler records no kernel at all (no CUPTI)."""
+    from torch.profiler import ProfilerActivity, profile
+    fn()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+        fn()
+        torch.cuda.synchronize()
+    names = [e.key for e in p.key_averages()]
+    return not any("kernel" in n for n in names) or any(part in n for n in names)

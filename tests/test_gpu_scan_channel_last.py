@@ -7,6 +7,7 @@ either side of a tie, and next to zero by the fp32 error of sums whose terms can
 import pytest
 import torch
 
+from helpers import launched
 from quamba_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
@@ -48,14 +49,6 @@ def _channel_last(c, workspace=True):
     return out, xs, fin
 
 
-def _kernel_of(fn):
-    from torch.profiler import ProfilerActivity, profile
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        fn()
-        torch.cuda.synchronize()
-    return [e.key for e in p.key_averages() if "sscan_cl" in e.key]
-
-
 def _close(got, want):
     y, xs, fin = got
     wy, wxs = want
@@ -74,8 +67,7 @@ def _close(got, want):
     (10, 1024, 2050, "<4, false>"), (1, 12288, 39, "<4, false>"), (1, 1536, 4100, "<4, true>"), (2, 100, 32, "<4, true>"), (3, 1000, 515, "<4, true>")])
 def test_each_form_against_the_sequence_last_kernel(B, d, L, kernel):
     c = _inputs(B, d, L)
-    names = _kernel_of(lambda: _channel_last(c))
-    assert any(kernel in n for n in names), names
+    assert launched(lambda: _channel_last(c), "sscan_cl_wide_kernel" if kernel == "wide" else "sscan_cl_kernel" + kernel)
     _close(_channel_last(c), _sequence_last(c))
 
 
@@ -88,8 +80,7 @@ def test_without_gate_skip_or_bias(B, d, L, z, D, bias):
 
 def test_without_workspace_the_rows_run_in_waves():
     c = _inputs(160, 512, 45, 2)
-    names = _kernel_of(lambda: _channel_last(c, False))
-    assert any("<1, false>" in n for n in names), names
+    assert launched(lambda: _channel_last(c, False), "sscan_cl_kernel<1, false>")
     _close(_channel_last(c, False), _sequence_last(c))
 
 

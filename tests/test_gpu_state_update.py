@@ -3,6 +3,7 @@ and against the CTA-tile kernel, with what a head shares and what a row has of i
 import pytest
 import torch
 
+from helpers import launched
 from oracle import update as oupd
 from quamba_b200 import _lib, ops
 
@@ -53,18 +54,8 @@ def _device(c):
     return y, st
 
 
-def _kernel_of(fn):
-    from torch.profiler import ProfilerActivity, profile
-    fn()
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        fn()
-        torch.cuda.synchronize()
-    return [e.key for e in p.key_averages() if "sscan_update" in e.key]
-
-
 def _check(c, kernel):
-    assert any(kernel in k for k in _kernel_of(lambda: _device(c))), "another kernel took the call"
+    assert launched(lambda: _device(c), kernel), "another kernel took the call"
     st, args = _args(c, lambda t: t)
     y_ref, _ = (oupd.quamba2_sscan_update if c["grouped"] else oupd.quant_sscan_update)(st, *args)
     y, got = _device(c)
