@@ -77,6 +77,7 @@ PyObject* conv1_update(const Args& a) {
   const int64_t batch = x.size(0), dim = x.size(1), width = w.size(-1);
   need(st.dim() == 3 && st.size(0) == batch && st.size(1) == dim && st.size(2) == width, "conv_state must have shape (batch, dim, width)");
   need(w.dim() == 2 && w.size(0) == dim, "weight must have shape (dim, width)");
+  on_gpu(bias, "bias");
   Device dev(x);
   Tensor out = dev.empty({batch, dim}, at::kChar);
   qb_conv1d_update_args s{};
@@ -201,6 +202,9 @@ PyObject* sscan_fwd(const Args& a) {
     sp[i] = f32(t);
   }
   const Tensor zs = a.opt_tensor(14), Ds = a.opt_tensor(12), bs = a.opt_tensor(16);
+  on_gpu(D, "D"); on_gpu(bias, "delta_bias");
+  if (Ds.defined()) cuda_f32(Ds, "scale_D");
+  if (bs.defined()) cuda_f32(bs, "scale_delta_bias");
   if (z.defined()) {
     cuda_i8(z, "z");
     need(z.sizes() == u.sizes() && (z.stride(-1) == 1 || z.size(-1) == 1), "z must match u");
@@ -245,6 +249,8 @@ PyObject* sscan_update(const Args& a) {
   const int64_t groups = B.size(1), batch = st.size(0), nh = st.size(1), dim = st.size(2), n = st.size(3);
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
   cuda_i8(st, "state"); cuda_i8(x, "q_x");
+  on_gpu(dt, "q_dt"); on_gpu(A, "q_A_log"); on_gpu(B, "q_B"); on_gpu(C, "q_C"); on_gpu(D, "q_D"); on_gpu(z, "q_z"); on_gpu(bias, "dt_bias");
+  on_gpu(hgr, "x_head_group_range"); on_gpu(dgr, "x_dim_group_range");
   cuda_f32(xs, "x_scales"); cuda_f32(ss, "ssm_state_scale"); cuda_f32(a.tensor(6), "dt_scale"); cuda_f32(a.tensor(8), "A_log_scale");
   cuda_f32(a.tensor(11), "B_scale"); cuda_f32(a.tensor(13), "C_scale");
   need(is(x, {batch, nh, dim}), "q_x must have shape (batch, nheads, dim)");
@@ -280,8 +286,8 @@ PyObject* sscan_update(const Args& a) {
   s.state = i8(st); s.x = i8(x); s.dt = i8(dt); s.A_log = i8(A); s.Bm = i8(B); s.Cm = i8(C); s.D = i8(D); s.z = i8(z);
   s.dt_bias = bias.defined() ? bias.data_ptr() : nullptr;
   s.x_scales = f32(xs); s.dt_scale = f32(a.tensor(6)); s.A_scale = f32(a.tensor(8)); s.state_scale = f32(ss); s.B_scale = f32(Bs); s.C_scale = f32(Cs);
-  s.D_scale = D.defined() ? f32(a.tensor(15)) : nullptr; s.z_scale = z.defined() ? f32(a.tensor(17)) : nullptr;
-  s.dt_bias_scale = bias.defined() && !half ? f32(bias_s) : nullptr;
+  s.D_scale = D.defined() ? scale_of(a.tensor(15), "D_scale") : nullptr; s.z_scale = z.defined() ? scale_of(a.tensor(17), "z_scale") : nullptr;
+  s.dt_bias_scale = bias.defined() && !half ? scale_of(bias_s, "dt_bias_scale") : nullptr;
   s.head_group_range = i32(hgr); s.dim_group_range = i32(dgr); s.out = out.data_ptr();
   s.state_sb = st.stride(0); s.state_sh = st.stride(1); s.state_sp = st.stride(2);
   s.x_sb = x.stride(0); s.x_sh = x.stride(1); s.dt_sb = dt.stride(0); s.dt_sh = dt.stride(1); s.dt_sp = dt.stride(2);
@@ -310,6 +316,7 @@ PyObject* ssd(const Args& a) {
   const int64_t batch = x.size(0), len = x.size(1), nh = x.size(2), hd = x.size(3), groups = B.size(2), n = B.size(3);
   need(groups > 0 && nh % groups == 0, "nheads must be divisible by ngroups");
   cuda_i8(x, "q_x"); cuda_i8(B, "q_B"); cuda_i8(dt, "q_dt"); cuda_i8(A, "q_A_log"); cuda_i8(C, "q_C");
+  on_gpu(D, "q_D"); on_gpu(z, "q_z"); on_gpu(bias, "dt_bias"); on_gpu(hgr, "x_head_group_range"); on_gpu(dgr, "x_dim_group_range");
   cuda_f32(xs, "x_scales"); cuda_f32(ss, "ssm_state_scale"); cuda_f32(a.tensor(5), "dt_scale"); cuda_f32(a.tensor(7), "A_log_scale");
   cuda_f32(Bs, "B_scale"); cuda_f32(Cs, "C_scale");
   auto is = [](const Tensor& t, std::initializer_list<int64_t> v) { return t.sizes() == at::IntArrayRef(v.begin(), v.size()); };
@@ -348,7 +355,7 @@ PyObject* ssd(const Args& a) {
   qb_ssd_args s{};
   s.x = i8(x); s.dt = i8(dt); s.Bm = i8(B); s.Cm = i8(C); s.A_log = i8(A); s.D = i8(D); s.z = i8(z); s.dt_bias = bias.defined() ? bias.data_ptr() : nullptr;
   s.x_scales = f32(xs); s.dt_scale = f32(a.tensor(5)); s.A_scale = f32(a.tensor(7)); s.B_scale = f32(Bs); s.C_scale = f32(Cs);
-  s.D_scale = D.defined() ? f32(a.tensor(15)) : nullptr; s.z_scale = z.defined() ? f32(a.tensor(17)) : nullptr; s.ssm_state_scale = f32(ss);
+  s.D_scale = D.defined() ? scale_of(a.tensor(15), "D_scale") : nullptr; s.z_scale = z.defined() ? scale_of(a.tensor(17), "z_scale") : nullptr; s.ssm_state_scale = f32(ss);
   s.head_group_range = i32(hgr); s.dim_group_range = i32(dgr); s.out = out.data_ptr(); s.final_states = i8(fin); s.workspace = ws.data_ptr(); s.workspace_bytes = wsb;
   s.x_sb = x.stride(0); s.x_sl = x.stride(1); s.x_sh = x.stride(2); s.dt_sb = dt.stride(0); s.dt_sl = dt.stride(1);
   s.B_sb = B.stride(0); s.B_sl = B.stride(1); s.B_sg = B.stride(2); s.C_sb = C.stride(0); s.C_sl = C.stride(1); s.C_sg = C.stride(2);
@@ -446,7 +453,7 @@ void check_norm(const Tensor& x, const Tensor& w, const Tensor& bias) {
   need(x.is_cuda() && x.scalar_type() == at::kHalf && x.dim() == 2, "x must be a 2-D float16 CUDA tensor");
   need(x.stride(-1) == 1, "x must be contiguous in its last dim");
   const int64_t n = x.size(1);
-  need(w.is_cuda(), "weight must be a CUDA tensor");
+  on_gpu(w, "weight"); on_gpu(bias, "bias");
   need(w.dim() == 1 && w.size(0) == n && w.stride(0) == 1 && w.scalar_type() == at::kHalf, "weight must be fp16 (N,)");
   if (bias.defined()) need(bias.dim() == 1 && bias.size(0) == n && bias.stride(0) == 1 && bias.scalar_type() == at::kHalf, "bias must be fp16 (N,)");
 }
@@ -465,6 +472,7 @@ PyObject* norm_fwd(const Args& a) {
   check_norm(x, w, bias);
   const int64_t m = x.size(0), n = x.size(1);
   int code = a.integer(6);
+  on_gpu(res, "residual");
   if (res.defined()) {
     need(res.sizes() == x.sizes() && res.stride(-1) == 1, "residual must have the shape of x");
     need(res.scalar_type() == at::kHalf || res.scalar_type() == at::kFloat, "residual must be float16 or float32");

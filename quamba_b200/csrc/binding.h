@@ -55,6 +55,13 @@ inline void cuda_i8(const Tensor& t, const char* name) {
 inline void cuda_f32(const Tensor& t, const char* name) {
   if (!t.is_cuda() || t.scalar_type() != at::kFloat) throw std::runtime_error(std::string(name) + " must be a float32 CUDA tensor");
 }
+inline void on_gpu(const Tensor& t, const char* name) {      // nothing given passes
+  if (t.defined() && !t.is_cuda()) throw std::runtime_error(std::string(name) + " must be a CUDA tensor");
+}
+inline const float* scale_of(const Tensor& t, const char* name) {
+  cuda_f32(t, name);
+  return static_cast<const float*>(t.data_ptr());
+}
 inline Tensor contiguous(const Tensor& t) {
   if (t.is_contiguous()) return t;
   const NoGil released;

@@ -62,6 +62,7 @@ Mod Mod::child(PyObject* name, PyTypeObject* type) const {
 }
 
 void Conv2::check() {
+  on_gpu(bias, "bias"); on_gpu(hgr, "x_head_group_range"); on_gpu(dgr, "x_dim_group_range");
   cuda_f32(out_scale[0], "x_scales"); cuda_f32(out_scale[1], "B_scales"); cuda_f32(out_scale[2], "C_scales");
   if (hgr.defined() && dgr.defined()) {
     need(hgr.scalar_type() == at::kInt && dgr.scalar_type() == at::kInt, "group ranges must be int32");

@@ -249,3 +249,23 @@ def test_mamba1_decode_against_the_module_walk(weights, batch):
     diff = (sa.int() - sb.int()).abs()
     assert diff.max() <= 1 and (diff != 0).float().mean() <= 2e-3
     assert (ya.float() - yb.float()).norm() <= 0.02 * yb.float().norm()
+
+
+@pytest.mark.parametrize("decode", [False, True])
+@pytest.mark.parametrize("family,buffers", [
+    ("mamba2", ("conv1d.bias", "conv1d.x_head_group_range", "conv1d.x_out_scales", "qchunk_scan.D", "qchunk_scan.dt_bias", "qchunk_scan.x_dim_group_range",
+                "qchunk_scan.ssm_state_scale")),
+    ("mamba1", ("conv1d.bias", "selective_scan.D", "selective_scan.dt_bias", "selective_scan.D_scale"))])
+def test_a_buffer_left_on_the_cpu_is_refused(family, buffers, decode):
+    layer = _layer("w4", True) if family == "mamba2" else _mamba1_layer("w4")
+    for path in buffers:
+        part, name = path.split(".")
+        mod = getattr(layer.mixer, part)
+        old = getattr(mod, name)
+        setattr(mod, name, old.cpu())
+        with pytest.raises(RuntimeError, match="CUDA"):
+            _call(layer, 2, 1 if decode else 5, decode)
+        setattr(mod, name, old)
+    h = torch.zeros(2, 1 if decode else 5, 256, device="cuda", dtype=torch.float16)
+    with pytest.raises(RuntimeError, match="CUDA"):
+        layer(h, torch.zeros(h.shape))
