@@ -8,6 +8,8 @@
 #include <stdio.h>
 #include <stdarg.h>
 
+#include <atomic>
+
 #include "../../include/quamba_b200.h"
 
 namespace qb {
@@ -112,16 +114,19 @@ int sm_count();         // multiprocessors the kernels size their grids for: the
 int device_sm_count();  // multiprocessor count of the current device (cached per device)
 
 // One-time-per-device guard for cudaFuncSetAttribute calls: kernel attributes belong to a device, so a process that
-// drives several GPUs must set them on each.  Returns true the first time it is asked about the current device.
-// (Two host threads asking at once may both get true: the attribute is then set twice to the same value, which is fine.)
+// drives several GPUs must set them on each.  A device counts as done once f() has returned, never before: a second host
+// thread asking meanwhile runs f() as well (the same values are then set twice, which is fine) instead of launching a kernel
+// that may not have its shared memory yet.
 struct PerDeviceOnce {
-  bool done[64] = {};
-  bool first() {
+  std::atomic<bool> done[64] = {};
+  template <typename F>
+  int run(F f) {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return true;
-    if (done[dev]) return false;
-    done[dev] = true;
-    return true;
+    const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    if (known && done[dev].load(std::memory_order_acquire)) return QB_OK;
+    const int rc = f();
+    if (known && rc == QB_OK) done[dev].store(true, std::memory_order_release);
+    return rc;
   }
 };
 

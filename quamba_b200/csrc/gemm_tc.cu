@@ -604,7 +604,11 @@ int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int 
   const size_t ring = std::max<size_t>((size_t)ts.stages * ts.stage_bytes, splits > 1 ? (size_t)ts.a_rows * (bn * 4 + 16) : 0);
   ts.ring_bytes = (int)ceil_div((int64_t)ring, 1024) * 1024;
   static PerDeviceOnce attr;
-  if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_kernel<kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+  rc = attr.run([]() -> int {
+    QB_CUDA_OK(cudaFuncSetAttribute(gemm_s8_kernel<kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+    return QB_OK;
+  });
+  if (rc != QB_OK) return rc;
   const size_t smem = (size_t)ts.ring_bytes + kFixedSmem;
   const int group = kPair ? 2 : splits;
   const unsigned grid = (unsigned)(std::min<int64_t>(tiles, sm_count() / group) * group);
@@ -618,10 +622,10 @@ int launch_gemm(const int8_t* A, int64_t lda, const int8_t* W, int64_t ldw, int 
 }
 
 int cluster_capacity(int splits) {
-  static int cached[64][9] = {};
+  static std::atomic<int> cached[64][9] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
-  int& c = cached[dev][splits];
+  int c = cached[dev][splits].load(std::memory_order_relaxed);
   if (c == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)splits * 64);
@@ -640,6 +644,7 @@ int cluster_capacity(int splits) {
       n = 0;
     }
     c = n > 0 ? n * splits : -1;
+    cached[dev][splits].store(c, std::memory_order_relaxed);
   }
   return std::min(c, sm_count());
 }
@@ -682,7 +687,11 @@ extern "C" int qb_i8_mma_peak(int groups, int repeats, void* stream, double* top
   QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "device status word unavailable");
   static PerDeviceOnce attr;
   constexpr int smem = kPeakBytes + 1024 + 256;
-  if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(i8_mma_peak_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int rc = attr.run([]() -> int {
+    QB_CUDA_OK(cudaFuncSetAttribute(i8_mma_peak_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return QB_OK;
+  });
+  if (rc != QB_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   cudaEvent_t e0, e1;
   QB_CUDA_OK(cudaEventCreate(&e0));

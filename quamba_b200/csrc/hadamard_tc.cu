@@ -316,7 +316,11 @@ int launch_one(const qb_hadamard_quant_args* a, const unsigned long long* masks,
   if (rc != QB_OK) return rc;
   auto kern = hadamard_tc_kernel<S, SPAD, R>;
   static PerDeviceOnce attr_done;
-  if (attr_done.first()) QB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  const int attr_rc = attr_done.run([&]() -> int {
+    QB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    return QB_OK;
+  });
+  if (attr_rc != QB_OK) return attr_rc;
   int* status = device_status_ptr();
   QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "hadamard: device status word unavailable");
   const int64_t units = ceil_div(a->rows, R);

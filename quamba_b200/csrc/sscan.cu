@@ -684,7 +684,11 @@ template <bool kGrouped, bool kTied, int kRows>
 int launch_update_warp(const qb_sscan_update_args& a, int* status, cudaStream_t st) {
   constexpr int smem = 8 * kWSlots * kRows * 128;
   static PerDeviceOnce attr;
-  if (attr.first()) QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_warp_kernel<kGrouped, kTied, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int rc = attr.run([]() -> int {
+    QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_warp_kernel<kGrouped, kTied, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return QB_OK;
+  });
+  if (rc != QB_OK) return rc;
   const int tiles = (int)((int64_t)a.batch * a.nheads * a.headdim / kRows);
   const dim3 grid((unsigned)std::min<int64_t>(ceil_div(tiles, 8), (int64_t)sm_count() * 2));
   launch_dependent(sscan_update_warp_kernel<kGrouped, kTied, kRows>, grid, dim3(256), smem, st, a, tiles, status);
@@ -1028,12 +1032,14 @@ extern "C" int qb_sscan_update(const qb_sscan_update_args* a, void* stream) {
 #define QB_UPD_LAUNCH(L)                                                                                           \
   do {                                                                                                             \
     static PerDeviceOnce attr_done; /* static + dynamic shared memory exceeds 48 KB for small dstate */          \
-    if (attr_done.first()) {                                                                                       \
+    const int attr_rc = attr_done.run([]() -> int {                                                                         \
       QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_bulk_kernel<L, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));   \
       QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_bulk_kernel<L, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));    \
       QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_bulk_kernel<L, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));  \
       QB_CUDA_OK(cudaFuncSetAttribute(sscan_update_bulk_kernel<L, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536));   \
-    }                                                                                                              \
+      return QB_OK;                                                                                           \
+    });                                                                                                            \
+    if (attr_rc != QB_OK) return attr_rc;                                                                          \
     if (tied && !grp) launch_dependent(sscan_update_bulk_kernel<L, true, false>, dim3(grid), dim3(256), smem, st, *a, tiles, tiles_per_cta, status);      \
     else if (tied && grp) launch_dependent(sscan_update_bulk_kernel<L, true, true>, dim3(grid), dim3(256), smem, st, *a, tiles, tiles_per_cta, status);   \
     else if (!grp) launch_dependent(sscan_update_bulk_kernel<L, false, false>, dim3(grid), dim3(256), smem, st, *a, tiles, tiles_per_cta, status);        \

@@ -453,8 +453,11 @@ int launch(const qb_sscan_fwd_args& a, int warps, int seg_len, cudaStream_t st) 
   const dim3 grid((unsigned)(kSeg ? groups : ceil_div(groups, warps)), (unsigned)a.batch);
   const size_t smem = (size_t)warps * (2 * kG * 32 + (kSeg ? (kN / kLanes + 1) * 32 : 0)) * sizeof(float);
   static PerDeviceOnce attr;
-  if (attr.first())
+  const int rc = attr.run([]() -> int {
     QB_CUDA_OK(cudaFuncSetAttribute(sscan_cl_kernel<kLanes, kSeg>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    return QB_OK;
+  });
+  if (rc != QB_OK) return rc;
   launch_dependent(sscan_cl_kernel<kLanes, kSeg>, grid, dim3((unsigned)warps * 32), smem, st, a, seg_len, early_overlap() ? 1 : 0);
   QB_LAUNCH_OK("sscan_cl_kernel");
   return QB_OK;
